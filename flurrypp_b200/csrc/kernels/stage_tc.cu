@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(128) k_elem_tc(ElemArgsT<float> a, const float
   constexpr int NS = T::NS, NFP = T::NFP, NF = T::NF, EB = T::EB, ROW = T::ROW;
   constexpr int NSp = T::NSp, K1p = T::K1p, K2p = T::K2p, K3p = T::K3p;
   extern __shared__ __align__(128) unsigned char smem_bytes[];
-  float *sm = reinterpret_cast<float *>((reinterpret_cast<uintptr_t>(smem_bytes) + 127) & ~uintptr_t(127));
+  float *sm = reinterpret_cast<float *>(smem_align128(smem_bytes));
   float *sOps = sm + T::O_OPS;
   float *sAh = sm + T::O_AH, *sAl = sm + T::O_AL;
   float *sU = sm + T::O_U, *sU0 = sm + T::O_U0, *sAcc = sm + T::O_ACC, *sCmp = sm + T::O_CMP;

@@ -155,7 +155,7 @@ __device__ __forceinline__ void two_sum(float a, float b, float &s, float &e) {
 // wavefronts were such conflicts).
 template <int NF, typename R>
 __device__ __forceinline__ int half_order(const R *p) {
-  return (int)((reinterpret_cast<uintptr_t>(p) >> 7) & 1);
+  return (int)((smem_u32(p) >> 7) & 1);
 }
 template <int NF, typename R>
 __device__ __forceinline__ void ldp(const R *p, R (&v)[NF]) {
@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(Tm<ND, P, R, V, VISC>::NT, Tm<ND, P, R, V, VIS
   };
   extern __shared__ __align__(128) unsigned char smem_bytes[];
   // tiles start on 128-byte boundaries relative to an aligned base
-  R *smem = reinterpret_cast<R *>((reinterpret_cast<uintptr_t>(smem_bytes) + 127) & ~uintptr_t(127));
+  R *smem = reinterpret_cast<R *>(smem_align128(smem_bytes));
   R *sU = smem + T::O_U;
   R *sU0 = smem + T::O_U0;  // not in the lean tile set
   R *sAcc = smem + T::O_ACC;
@@ -806,7 +806,7 @@ __global__ void __launch_bounds__(Tg2<ND, P, R>::NT) k_grad_tma(int E, TpTablesT
   using T = Tg2<ND, P, R>;
   constexpr int N = T::N, NF = T::NF, NS = T::NS, NFP = T::NFP, EB = T::EB, NT = T::NT, ROW = T::ROW;
   extern __shared__ __align__(128) unsigned char smem_bytes[];
-  R *smem = reinterpret_cast<R *>((reinterpret_cast<uintptr_t>(smem_bytes) + 127) & ~uintptr_t(127));
+  R *smem = reinterpret_cast<R *>(smem_align128(smem_bytes));
   R *sU = smem + T::O_U;
   R *sC = smem + T::O_C;      // [NFP][ROW] LDG jumps
   R *sJ = smem + T::O_J;      // [ND][NS][EB*ND]

@@ -12,6 +12,14 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
 
+// The first 128-byte boundary of a dynamic shared-memory array, as an offset
+// from the array: rounding the generic address up instead would lose the
+// address space, and every access through the result would compile to a
+// generic load or store in place of a shared-memory one.
+__device__ __forceinline__ unsigned char *smem_align128(unsigned char *smem) {
+  return smem + ((128u - (smem_u32(smem) & 127u)) & 127u);
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
