@@ -35,12 +35,45 @@ struct Phys {
   int riemannType;    // 0 Rusanov, 1 Roe (2-D interior faces only)
 };
 
+// 1/x and sqrt(x) of a positive state value by Newton's method from the
+// hardware's approximation (relative error below 2^-20 in FP64, 2^-22 in
+// FP32; each step squares the error), the last step formed as a residual
+// correction, which leaves at most the last bit open.  Without the general
+// functions' branches for subnormal and huge arguments the chains of a
+// point's states overlap: they are the longest of a flux evaluation.  A root
+// below 1e-290 (FP32 1e-36), which no state reaches, is taken as zero; a
+// non-finite argument gives a non-finite result.
+__device__ __forceinline__ double recip(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = fma(y, fma(-x, y, 1.0), y);
+  return fma(y, fma(-x, y, 1.0), y);
+}
+__device__ __forceinline__ float recip(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return fmaf(y, fmaf(-x, y, 1.0f), y);
+}
+__device__ __forceinline__ double root(double x) {
+  double r;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  r = fma(0.5 * r, fma(-x * r, r, 1.0), r);
+  const double s = x * r, h = 0.5 * r;
+  return x > 1e-290 ? fma(h, fma(-s, s, x), s) : 0.0;
+}
+__device__ __forceinline__ float root(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  const float s = x * r, h = 0.5f * r;
+  return x > 1e-36f ? fmaf(h, fmaf(-s, s, x), s) : 0.0f;
+}
+
 // Euler flux F[d][k] (reference: src/flux.cpp:37-76).
 template <int ND, typename R>
 __device__ __forceinline__ void inviscid_flux(const R *U, R F[ND][ND + 2], R gam) {
   if (ND == 2) {
     R rho = U[0];
-    R ri = R(1.0) / rho;
+    R ri = recip(rho);
     R u = U[1] * ri;
     R v = U[2] * ri;
     R E = U[3];
@@ -51,7 +84,7 @@ __device__ __forceinline__ void inviscid_flux(const R *U, R F[ND][ND + 2], R gam
     F[0][3] = (E + p) * u;      F[1][3] = (E + p) * v;
   } else {
     R rho = U[0];
-    R ri = R(1.0) / rho;
+    R ri = recip(rho);
     R u = U[1] * ri;
     R v = U[2] * ri;
     R w = U[3] * ri;
@@ -73,7 +106,7 @@ struct Prim {
   R rinv;
   __device__ __forceinline__ Prim(const R *U, R gam) {
     rho = U[0];
-    rinv = R(1.0) / rho;  // one reciprocal per state instead of a division per term
+    rinv = recip(rho);  // one reciprocal per state instead of a division per term
 #pragma unroll
     for (int d = 0; d < ND; d++) vel[d] = U[d + 1] * rinv;
     E = U[ND + 1];
@@ -114,14 +147,15 @@ __device__ __forceinline__ R rusanov(const R *UL, const R *UR, const R *n, R gam
   }
   R csqL = fmax(gam * L.p * L.rinv, R(0.0));
   R csqR = fmax(gam * Rt.p * Rt.rinv, R(0.0));
-  R eigL = fabs(vnL) + sqrt(csqL);
-  R eigR = fabs(vnR) + sqrt(csqR);
+  const R cL = root(csqL), cR = root(csqR);
+  R eigL = fabs(vnL) + cL;
+  R eigR = fabs(vnR) + cR;
   R eig = fmax(eigL, eigR);
 #pragma unroll
   for (int i = 0; i < NF; i++) Fn[i] = R(0.5) * (tL[i] + tR[i] - eig * (UR[i] - UL[i]));
   // the wave speed kept for the time step is relative to the grid velocity
   // on a moving mesh (face.cpp:366-371; vgn is zero on a static one)
-  return fmax(fabs(vnL - vgn) + sqrt(csqL), fabs(vnR - vgn) + sqrt(csqR));
+  return fmax(fabs(vnL - vgn) + cL, fabs(vnR - vgn) + cR);
 }
 
 // Roe flux with entropy fix, 2-D (reference: src/face.cpp:376-495).
@@ -302,12 +336,13 @@ template <int ND, typename R>
 __device__ __forceinline__ void viscous_flux(const R *U, const R gradU[ND][ND + 2], const Phys &ph,
                                              R Fvis[ND][ND + 2]) {
   R rho = U[0];
-  R u = U[1] / rho;
-  R v = U[2] / rho;
-  R e = U[ND + 1] / rho - R(0.5) * (u * u + v * v);
+  const R ri = recip(rho);  // multiplied: 16 divisions by rho otherwise
+  R u = U[1] * ri;
+  R v = U[2] * ri;
+  R e = U[ND + 1] * ri - R(0.5) * (u * u + v * v);
   R w;
   if (ND == 3) {
-    w = U[3] / rho;
+    w = U[3] * ri;
     e -= R(0.5) * (w * w);
   } else {
     w = R(0.);
@@ -330,17 +365,17 @@ __device__ __forceinline__ void viscous_flux(const R *U, const R gradU[ND][ND + 
     R rt_ratio = (R(ph.gamma) - R(1.0)) * e / R(ph.rt_inf);
     mu *= pow(rt_ratio, R(1.5)) * (R(1.) + R(ph.c_sth)) / (rt_ratio + R(ph.c_sth));
   }
-  R du_dx = (dRhoU_dx - dRho_dx * u) / rho;
-  R du_dy = (dRhoU_dy - dRho_dy * u) / rho;
-  R dv_dx = (dRhoV_dx - dRho_dx * v) / rho;
-  R dv_dy = (dRhoV_dy - dRho_dy * v) / rho;
+  R du_dx = (dRhoU_dx - dRho_dx * u) * ri;
+  R du_dy = (dRhoU_dy - dRho_dy * u) * ri;
+  R dv_dx = (dRhoV_dx - dRho_dx * v) * ri;
+  R dv_dy = (dRhoV_dy - dRho_dy * v) * ri;
   R du_dz = R(0), dv_dz = R(0), dw_dx = R(0), dw_dy = R(0), dw_dz = R(0);
   if (ND == 3) {
-    du_dz = (dRhoU_dz - dRho_dz * u) / rho;
-    dv_dz = (dRhoV_dz - dRho_dz * v) / rho;
-    dw_dx = (dRhoW_dx - dRho_dx * w) / rho;
-    dw_dy = (dRhoW_dy - dRho_dy * w) / rho;
-    dw_dz = (dRhoW_dz - dRho_dz * w) / rho;
+    du_dz = (dRhoU_dz - dRho_dz * u) * ri;
+    dv_dz = (dRhoV_dz - dRho_dz * v) * ri;
+    dw_dx = (dRhoW_dx - dRho_dx * w) * ri;
+    dw_dy = (dRhoW_dy - dRho_dy * w) * ri;
+    dw_dz = (dRhoW_dz - dRho_dz * w) * ri;
   }
   R dK_dx, dK_dy, dK_dz;
   if (ND == 2) {
@@ -352,11 +387,11 @@ __device__ __forceinline__ void viscous_flux(const R *U, const R gradU[ND][ND + 
     dK_dy = R(0.5) * (u * u + v * v + w * w) * dRho_dy + rho * (u * du_dy + v * dv_dy + w * dw_dy);
     dK_dz = R(0.5) * (u * u + v * v + w * w) * dRho_dz + rho * (u * du_dz + v * dv_dz + w * dw_dz);
   }
-  R de_dx = (dE_dx - dK_dx - dRho_dx * e) / rho;
-  R de_dy = (dE_dy - dK_dy - dRho_dy * e) / rho;
+  R de_dx = (dE_dx - dK_dx - dRho_dx * e) * ri;
+  R de_dy = (dE_dy - dK_dy - dRho_dy * e) * ri;
   R de_dz = R(0);
-  if (ND == 3) de_dz = (dE_dz - dK_dz - dRho_dz * e) / rho;
-  R diag = (du_dx + dv_dy + dw_dz) / R(3.0);
+  if (ND == 3) de_dz = (dE_dz - dK_dz - dRho_dz * e) * ri;
+  R diag = (du_dx + dv_dy + dw_dz) * R(1.0 / 3.0);
   R tauxx = R(2.0) * mu * (du_dx - diag);
   R tauyy = R(2.0) * mu * (dv_dy - diag);
   R tauxy = mu * (du_dy + dv_dx);
@@ -371,7 +406,7 @@ __device__ __forceinline__ void viscous_flux(const R *U, const R gradU[ND][ND + 
     }
     tauzz = R(2.0) * mu * (dw_dz - diag);
   }
-  R kq = (mu / R(ph.prandtl)) * R(ph.gamma);
+  R kq = (mu * recip(R(ph.prandtl))) * R(ph.gamma);
   Fvis[0][0] = R(0.0);
   Fvis[0][1] = -tauxx;
   Fvis[0][2] = -tauxy;
