@@ -281,6 +281,15 @@ def elem_bytes(s, wbytes):
     return wbytes * E * (5 * nS * nF + 2 * nFp * nF + nd * nd * nS + nS)
 
 
+def stage_bytes(s, wbytes):
+    """Algorithmic bytes of one intermediate RK stage in one launch: read U, U0,
+    the running sum (3 nS nF), the neighbours' traces (nFp nF), metrics
+    (nDims^2 + 1) nS, normals and areas (nDims + 1) nFp, neighbour slots; write
+    U and the sum (2 nS nF) and the traces (nFp nF)."""
+    nS, nFp, nF, nd, E = s.nSpts, s.nFpts, s.nFields, s.nDims, s.nEles
+    return E * (wbytes * (5 * nS * nF + 2 * nFp * nF + (nd * nd + 1) * nS + (nd + 1) * nFp) + 4 * nFp)
+
+
 def kernel_ms(torch, stream, s, kernel, reps=20):
     s.bench_kernel(kernel, 2)
     return dev_ms(torch, stream, lambda: s.bench_kernel(kernel, reps)) / reps
@@ -295,11 +304,12 @@ def form_precision_tgv32(args, fb, torch, stream, dt):
     s.run(args.warmup)
     ms = dev_ms(torch, stream, lambda: s.run(args.steps))
     inf = s.info()
+    sm = kernel_ms(torch, stream, s, "stage")
     km = kernel_ms(torch, stream, s, "element_stage")
     fm = kernel_ms(torch, stream, s, "faces")
     peak, _ = measured_peak_hbm()
-    eb = elem_bytes(s, 4)
-    ach = eb / (km / 1e3) / 1e9
+    eb = stage_bytes(s, 4)
+    ach = eb / (sm / 1e3) / 1e9
     del s
     # error after 200 steps vs the plain form, same initial state and dt
     runs = {}
@@ -316,8 +326,8 @@ def form_precision_tgv32(args, fb, torch, stream, dt):
         "value": dof * nrk * args.steps / (ms / 1e3), "unit": METRIC, "ms_per_step": ms / args.steps,
         "dtype": "f32 (FP64 dt, metrics at setup, norms)",
         "tile_variant": inf.tile_variant, "elems_per_block": inf.elems_per_block,
-        "kernels_ms": {"element_stage": km, "faces": fm},
-        "roofline": {"bound": "hbm", "kernel": f"k_elem_tma<3, 3, float, {inf.tile_variant}>",
+        "kernels_ms": {"stage": sm, "two_kernel_form": {"element_stage": km, "faces": fm}},
+        "roofline": {"bound": "hbm", "kernel": "k_fused_stage<3, 3, float>",
                      "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
                      "algorithmic_bytes": eb},
         "error_vs_fp64": dict(steps=args.err_steps, **state_errors(runs[fb.FR_PREC_MIXED], runs[fb.FR_PREC_FP64])),
@@ -873,7 +883,7 @@ def main():
 
     # dominant kernels timed alone (same stream)
     kt = {}
-    for k in ("element_stage", "faces"):
+    for k in ("stage", "element_stage", "faces"):
         s.bench_kernel(k, 2)
         a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         reps = 20
@@ -965,17 +975,14 @@ def main():
         e2e = whole_job_rate(world, dof, nrk, args.e2e_steps, ms_e2e)
         e2e_copy_bound = whole_job_rate(world, dof, nrk, args.e2e_steps, ms_copy)
         peak, peak_kind = measured_peak_hbm()
-        # algorithmic bytes per launch of the element kernel (intermediate RK
-        # stage, FP64): per element read U, U0, acc, Fn (nFpts*nF), JGinv
-        # (nDims^2*nS), detJ (nS); write acc, U, U_fpts (nFpts*nF)
-        nS, nFp, nF, nd, E = s.nSpts, s.nFpts, s.nFields, s.nDims, s.nEles
-        elem_bytes = 8 * E * (5 * nS * nF + 2 * nFp * nF + nd * nd * nS + nS)
+        nF, nd = s.nFields, s.nDims
+        alg_bytes = stage_bytes(s, 8)
         inf = s.info()
         # face kernel: per face point read 2 slots, normal, dA L/R, U L/R;
         # write Fn L/R and the left wave speed
         nfp = inf.nFacePts
         face_bytes = nfp * (8 + 8 * nd + 16 + 2 * 8 * nF + 2 * 8 * nF + 8)
-        ach = elem_bytes / (kt["element_stage"] / 1e3) / 1e9
+        ach = alg_bytes / (kt["stage"] / 1e3) / 1e9
         out = {
             "metric": METRIC, "value": value, "unit": METRIC, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True,
@@ -987,14 +994,15 @@ def main():
                     "copy_bound": e2e_copy_bound, "frac_of_copy_bound": e2e / e2e_copy_bound},
             "gpu_launches": launches,
             "roofline": {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
-                         "traffic": profiled_traffic("traffic_bytes_per_launch"),
+                         "traffic": profiled_traffic("one_launch_traffic_bytes"),
                          "traffic_source": "profiles/fp64_stage_tgv32_p3.md (ncu, one launch)",
-                         "kernel": "k_elem_tma<3, 3>" if inf.tensor_kernels == 2 else "k_elem_tp<3, 3>",
+                         "kernel": "k_fused_stage<3, 3, double>",
                          "tile_variant": inf.tile_variant, "elems_per_block": inf.elems_per_block,
-                         "kernel_ms": kt["element_stage"], "algorithmic_bytes": elem_bytes,
+                         "kernel_ms": kt["stage"], "algorithmic_bytes": alg_bytes,
                          "peak_source": peak_kind},
-            "kernels_ms": {"element_stage": kt["element_stage"], "faces": kt["faces"],
-                           "faces_GBps": face_bytes / (kt["faces"] / 1e3) / 1e9},
+            "kernels_ms": {"stage": kt["stage"],
+                           "two_kernel_form": {"element_stage": kt["element_stage"], "faces": kt["faces"],
+                                               "faces_GBps": face_bytes / (kt["faces"] / 1e3) / 1e9}},
             "clocks": clk.summary(),
         }
         if world == 1 and not args.no_cpu_baseline:

@@ -110,7 +110,6 @@ struct fr_case {
   int nDims = 0, nF = 0, nS = 0, nFp = 0, E = 0, nPF = 0, nRK = 0;
   long long iter = 0;
   long long launches = 0;  // kernels launched (graph replays counted per kernel)
-  int graphKernels = 0;    // kernels in the captured step
   double hostDt = 0.0;
   bool stateSet = false;
   bool fptsFresh = false;  // U_fpts holds the extrapolation of U_spts
@@ -137,12 +136,11 @@ struct fr_case {
   unsigned int *devErr = nullptr;
   int EB = 1;
   frk::Phys ph{};
-  cudaGraphExec_t graph = nullptr;
-  // kRunChunk steps in one graph, for runs of at least that many steps (one
-  // graph launch instead of kRunChunk)
+  // step graphs by their number of steps (1 .. kRunChunk): a run is one
+  // launch per kRunChunk steps and one for the rest
   static constexpr int kRunChunk = 10;
-  cudaGraphExec_t graphK = nullptr;
-  int graphKernelsK = 0;
+  cudaGraphExec_t graphs[kRunChunk + 1] = {};
+  int graphKernels[kRunChunk + 1] = {};  // kernels in each
   bool ownStream = false;
   bool hostOnly = false;  // set up without a device: setup arrays only
   // P-multigrid (reference: multigrid.cpp:47-384): coarse levels share the
@@ -177,6 +175,31 @@ struct fr_case {
     float *tcOps = nullptr;     // 2-D tensor-core variant: operators in MMA layout
     std::vector<float> tuneMs;  // element-stage time per tile variant (autotuner)
   } f32;
+
+  // One-launch RK stages (kernels/stage_fused.cu) of inviscid static cases:
+  // thread-order copies of the metrics and the face table, the second trace
+  // buffer (stages read one and write the other; a step has an even number
+  // of stages, so it ends in U_fpts), the stage sums, the tensor maps.  The
+  // stages after the first work in the array `acc`, so U keeps the step's
+  // base state until the last one.
+  template <typename R>
+  struct FusedDev {
+    R *jg = nullptr, *rdet = nullptr, *nrm = nullptr, *X0 = nullptr, *S = nullptr, *Uf2 = nullptr;
+    frk::FusedArgsT<R> a;             // what every stage shares
+    CUtensorMap U, B, U0, Uf, Uf2m;
+  };
+  struct Fused {
+    bool on = false, tma = false;
+    int *nb = nullptr, *lineF = nullptr, *lineOf = nullptr;
+    FusedDev<double> d;
+    FusedDev<float> f;
+  } fz;
+  std::vector<double> hD, hE1, hEF, hLC;  // the 1-D operator tables (build_tp)
+  std::vector<int> hLineF, hLineOf;
+  // Fn_fpts is formed on demand after one-launch stages, from the traces of
+  // the last evaluation (fnOld: in the second trace buffer, else in U_fpts);
+  // fnPinned: a caller holds its device pointer, so every call refreshes it
+  bool fnStale = false, fnOld = false, fnPinned = false;
 
   // moving mesh (deck "motion" 1..5): the vertex law, the metrics rebuilt at
   // every RK stage and the chain-rule residual (kernels/motion.cu)
@@ -227,6 +250,7 @@ struct fr_case {
   // evaluation (boundFace::computeWallForce / computeMassFlux)
   bool boundary_monitors(int errorNorm, double *host11) {
     const int nB = ft.n - ft.nInterior;
+    ensure_fn();
     if (!monOut && (!alloc(monPart, (size_t)std::max(nB, 1) * 11) || !alloc(monOut, 11))) return false;
     if (!mixed) {
       frk::MonitorArgsT<double> a;
@@ -274,8 +298,7 @@ struct fr_case {
     if (cp.done) cudaEventDestroy(cp.done);
     if (cp.copy) cudaStreamDestroy(cp.copy);
     if (stream) cudaStreamSynchronize(stream);
-    if (graph) cudaGraphExecDestroy(graph);
-    if (graphK) cudaGraphExecDestroy(graphK);
+    drop_graphs();
     levels.clear();  // coarse levels use this case's stream: release them first
     for (auto &b : allocs) {
       if (b.fp32) note_fp32(b.p, b.bytes, false);
@@ -284,6 +307,12 @@ struct fr_case {
     if (ownStream && ownedStream) cudaStreamDestroy(ownedStream);
   }
   cudaStream_t ownedStream = nullptr;
+  void drop_graphs() {
+    for (auto &g : graphs) {
+      if (g) cudaGraphExecDestroy(g);
+      g = nullptr;
+    }
+  }
 
   int errCode = 0;  // the FR_ERR_* of the last fail()
   bool fail(int code, const std::string &m) {
@@ -527,6 +556,7 @@ struct fr_case {
     } else if (useTp && !opts.no_tma && (E * nF) % 4 == 0) {
       if (!autotune_tiles()) return false;
     }
+    if (!setup_fused()) return false;
     hostDt = in.dt;
     if (cudaMemcpyAsync(dt, &hostDt, sizeof(double), cudaMemcpyHostToDevice, stream) != cudaSuccess)
       return fail(FR_ERR_CUDA, "dt upload");
@@ -994,6 +1024,19 @@ struct fr_case {
         }
       }
     }
+    hD = D, hE1 = E1, hEF = EF, hLC = LC;
+    // lines by (dimension, transverse index): their end flux points, and the
+    // reverse map
+    const int nLines = nS / n;
+    hLineF.assign((size_t)nDims * nLines, 0);
+    hLineOf.assign(nFp, 0);
+    for (int pr : pair) {
+      const int f0 = pr & 0xffff, f1 = pr >> 16, d = fDn[f0], base = fBase[f0];
+      const int c = d == nDims - 1 ? base : d == 0 ? base / n : base % n + base / (n * n) * n;
+      hLineF[(size_t)d * nLines + c] = pr;
+      hLineOf[f0] = 2 * (d * nLines + c);
+      hLineOf[f1] = 2 * (d * nLines + c) + 1;
+    }
     double *dD, *dE1, *dEF, *dcV, *dLC;
     int *dfB, *dfD, *dfS, *dcF, *dLP;
     if (!upload(dD, D) || !upload(dE1, E1) || !upload(dEF, EF) || !upload(dfB, fBase) || !upload(dfD, fDn) ||
@@ -1197,6 +1240,149 @@ struct fr_case {
   bool build_tma(int v) {
     return build_maps<double>(tm, frk::tma_elems_per_block<double>(nDims, in.order, v), U, U0, acc, nullptr, Fn,
                               Ufpts, detJ, JGinv, detTma, jgTma, dUs, dUc, dUf);
+  }
+
+  // One-launch stages: inviscid static cases with tensor-product operators
+  // and an even number of stages, unless an option asks for another kernel.
+  bool setup_fused() {
+    const int n = in.order + 1, nLines = nS / n;
+    if (!useTp || in.viscous || in.motion || nRK % 2 != 0 || opts.no_tma || opts.tile_variant >= 0 ||
+        (long long)nFp * E >= (1LL << 30))
+      return true;
+    const int eb = mixed ? frk::fused_elems_per_block<float>(nDims, in.order)
+                         : frk::fused_elems_per_block<double>(nDims, in.order);
+    const size_t nBlk = (E + eb - 1) / eb, lanes = nBlk * nLines * eb;
+    std::vector<int> lines(hLineF);
+    lines.insert(lines.end(), hLineOf.begin(), hLineOf.end());
+    if (!upload(fz.lineF, lines)) return false;
+    fz.lineOf = fz.lineF + hLineF.size();
+    const bool ok = mixed ? setup_fused_as<float>(fz.f, lanes, eb, f32.U, f32.acc, f32.U0, f32.Ufpts, f32.JGinv,
+                                                  f32.detJ, f32.ft)
+                          : setup_fused_as<double>(fz.d, lanes, eb, U, acc, U0, Ufpts, JGinv, detJ, ft);
+    if (!ok) return false;
+    fz.on = true;
+    return cuda_ok("one-launch stage setup");
+  }
+  template <typename R>
+  bool setup_fused_as(FusedDev<R> &z, size_t lanes, int eb, R *u, R *b, R *u0, R *uf, const R *jgi, const R *det,
+                      const frk::FaceTableT<R> &table) {
+    const int n = in.order + 1;
+    const size_t nUf = (size_t)nFp * E * nF;
+    // one allocation for all of them: a small case's setup is mostly these calls
+    size_t total = 0;
+    auto take = [&](size_t count) {  // in R, on 256-byte boundaries
+      const size_t at = total;
+      total += (count + 255 / sizeof(R)) / (256 / sizeof(R)) * (256 / sizeof(R));
+      return at;
+    };
+    const size_t oJ = take(lanes * n * nDims * nDims), oR = take(lanes * n), oN = take(lanes * 2 * nDims * (nDims + 1)),
+                 oX = take(lanes * n * nF), oS = take(lanes * n * nF), oT = take(nUf),
+                 oB = take((lanes * 2 * nDims * sizeof(int) + sizeof(R) - 1) / sizeof(R));
+    R *pool = nullptr;
+    if (!alloc(pool, total)) return false;
+    z.jg = pool + oJ, z.rdet = pool + oR, z.nrm = pool + oN, z.X0 = pool + oX, z.S = pool + oS, z.Uf2 = pool + oT;
+    fz.nb = reinterpret_cast<int *>(pool + oB);
+    frk::launch_fused_pack<R>(nDims, in.order, E, jgi, det, table, fz.lineOf, z.jg, z.rdet, fz.nb, z.nrm, stream);
+    auto encode = tensor_map_encoder();
+    const CUtensorMapDataType ty = sizeof(R) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+    auto map = [&](CUtensorMap *m, void *p, int rows) {
+      cuuint64_t dims[2] = {(cuuint64_t)E * nF, (cuuint64_t)rows};
+      cuuint64_t str[1] = {(cuuint64_t)E * nF * sizeof(R)};
+      cuuint32_t box[2] = {(cuuint32_t)(eb * nF), (cuuint32_t)rows}, es[2] = {1, 1};
+      return encode(m, ty, 2, p, dims, str, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    // rows of a tensor map start on 16-byte boundaries (2-D always do)
+    fz.tma = encode && (size_t)E * nF * sizeof(R) % 16 == 0 && map(&z.U, u, nS) && map(&z.B, b, nS) &&
+             map(&z.U0, u0, nS) && map(&z.Uf, uf, nFp) && map(&z.Uf2m, z.Uf2, nFp);
+    if (!fz.tma && nDims == 2) return fail(FR_ERR_CUDA, "tensor map");
+    frk::FusedArgsT<R> &a = z.a;
+    a.E = E;
+    a.S = z.S;
+    a.X0 = z.X0;
+    a.jg = z.jg;
+    a.rdet = z.rdet;
+    a.nrm = z.nrm;
+    a.nb = fz.nb;
+    a.lineF = fz.lineF;
+    a.dt = dt;
+    a.eleDt = (in.dtType == 2 || perElementDt) ? eleDt : nullptr;
+    a.err = devErr;
+    a.ph = ph;
+    for (int i = 0; i < n * n; i++) a.D[i] = (R)hD[i];
+    for (int i = 0; i < 2 * n; i++) a.E1[i] = (R)hE1[i], a.EFn1[i] = (R)hEF[i], a.C[i] = (R)hLC[i];
+    return true;
+  }
+  bool fused_ok() const { return fz.on && cut.n == 0; }
+
+  // One stage: -1 the residual alone (divF_out), else stage `st` of a step.
+  // keepDivF / keepU0 / wave: the arrays a caller may look at after the call.
+  template <typename R>
+  void fused_launch(FusedDev<R> &z, int st, R *u, R *b, R *u0, R *uf, R *cmp, R *divOut, const R *source, bool keepU0,
+                    bool wave) {
+    frk::FusedArgsT<R> a = z.a;
+    frk::FusedMaps m;
+    const bool jameson = in.timeType >= 5;
+    const bool odd = st > 0 && st % 2 == 1;
+    a.first = st <= 0;
+    a.Uin = st <= 0 ? u : b;
+    m.in = st <= 0 ? z.U : z.B;
+    a.Ufin = odd ? z.Uf2 : uf;
+    a.divF = divOut;
+    a.src = source;
+    a.waveSp = wave ? wave_out() : nullptr;
+    if (st >= 0) {
+      const bool last = st == nRK - 1;
+      a.mode = last ? frk::FUSED_FINAL : frk::FUSED_STAGE;
+      a.Uout = last ? u : b;
+      m.out = last ? z.U : z.B;
+      a.Ufout = odd ? uf : z.Uf2;
+      m.tr = odd ? z.Uf : z.Uf2m;
+      a.keepU0 = keepU0 && st == 0;
+      a.U0keep = u0;
+      m.keep = z.U0;
+      a.comp = cmp;
+      a.timeAcc = last && !pmgCoarse ? timeAcc : nullptr;
+      if (jameson) {
+        if (last)
+          a.rkb = in.RKa[nRK];
+        else
+          a.rka = in.RKa[st + 1];
+      } else {
+        if (!last) a.rka = in.RKa[st + 1];
+        a.rkb = in.RKb[st];
+        a.saveS = !last;
+        a.loadS = st > 0;
+      }
+    }
+    frk::launch_fused_stage<R>(nDims, in.order, fz.tma, a, m, stream);
+    launches++;
+    fnStale = true;
+    fnOld = odd;
+  }
+  void fused_stage(int st, bool keepDivF, bool pmgSource, bool keepU0, bool wave) {
+    if (mixed)
+      fused_launch<float>(fz.f, st, f32.U, f32.acc, f32.U0, f32.Ufpts, f32.comp, keepDivF ? f32.divF[0] : nullptr,
+                          pmgSource ? src32 : nullptr, keepU0, wave);
+    else
+      fused_launch<double>(fz.d, st, U, acc, U0, Ufpts, nullptr, keepDivF ? divF[0] : nullptr,
+                           pmgSource ? src : nullptr, keepU0, wave);
+  }
+  // Fn_fpts of the last evaluation, where one-launch stages did not store it
+  // new traces of a state the caller changed: first Fn_fpts of the last
+  // evaluation, if it is still to be formed from the traces replaced here
+  void renew_traces() {
+    if (!fnOld) ensure_fn();
+    extrapolate();
+  }
+  void ensure_fn() {
+    if (!fnStale) return;
+    if (mixed)
+      frk::launch_faces_inviscid<float>(nDims, f32.ft, fnOld ? fz.f.Uf2 : f32.Ufpts, f32.Fn, nullptr, ph, stream);
+    else
+      frk::launch_faces_inviscid(nDims, ft, fnOld ? fz.d.Uf2 : Ufpts, Fn, nullptr, ph, stream);
+    launches++;
+    fnStale = false;
   }
 
   // The plain form's tile autotuner: the same timing as autotune_tiles on
@@ -1692,6 +1878,15 @@ struct fr_case {
     // the last element stage extrapolated the state it wrote; otherwise
     // (a new or restricted/prolonged state) extrapolate here
     if (!fptsFresh) extrapolate();
+    if (fused_ok() && !opts.debug_arrays) {
+      if (mixed)
+        fused_launch<float>(fz.f, -1, f32.U, f32.acc, f32.U0, f32.Ufpts, nullptr, f32.divF[step], nullptr, false, true);
+      else
+        fused_launch<double>(fz.d, -1, U, acc, U0, Ufpts, nullptr, divF[step], nullptr, false, true);
+      if (fnPinned) ensure_fn();
+      return cuda_ok("calc_residual");
+    }
+    fnStale = false;
     faces_pass();
     if (!mixed) {
       frk::ElemArgs a = elem_args();
@@ -1711,10 +1906,21 @@ struct fr_case {
     return cuda_ok("calc_residual");
   }
 
-  // solver::update (solver.cpp:319-363)
-  bool update_once(bool pmgSource) {
+  // solver::update (solver.cpp:319-363).  last: a caller can look at this
+  // step's divF_0, U0 and wave speeds (inside a run only the last step's can
+  // be seen); ownDivF: nothing overwrites divF_0 after this call
+  bool update_once(bool pmgSource, bool last = true, bool ownDivF = true) {
     if (mo.on) return update_motion(pmgSource);
     if (!fptsFresh) extrapolate();
+    if (fused_ok()) {
+      if (in.dtType != 0) calc_dt_dev();
+      for (int st = 0; st < nRK; st++)
+        fused_stage(st, st == 0 && last && ownDivF && !pmgCoarse, pmgSource, last && !pmgCoarse,
+                    st == nRK - 1 && (last || in.dtType != 0));
+      fptsFresh = true;
+      return cuda_ok("update");
+    }
+    fnStale = false;
     const bool jameson = in.timeType >= 5;
     for (int step = 0; step < nRK - 1; step++) {
       if (step == 0 && in.dtType != 0) calc_dt_dev();
@@ -1742,15 +1948,39 @@ struct fr_case {
   bool update(bool pmgSource) {
     if (!stateSet) return fail(FR_ERR_STATE, "no state set");
     iter++;
-    return update_once(pmgSource);
+    const bool ok = update_once(pmgSource);
+    if (fnPinned) ensure_fn();
+    return ok;
   }
 
   // one step of the driver loop: update, then the P-multigrid cycle when on
   // (reference: flurry.cpp:162-170)
-  bool step_once() {
-    if (!update_once(false)) return false;
-    if (in.PMG && !pmgCoarse && !levels.empty()) return pmg_cycle();
+  bool step_once(bool last = true) {
+    const bool cycle = in.PMG && !pmgCoarse && !levels.empty();
+    if (!update_once(false, last, !cycle)) return false;
+    if (cycle) return pmg_cycle();
     return true;
+  }
+
+  bool capture(int steps) {
+    if (!stream) return fail(FR_ERR_STATE, "graph capture needs a non-default stream");
+    cudaGraph_t g;
+    const long long saveIter = iter;
+    iter = 2;  // steady-state branch
+    if (cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+      iter = saveIter;
+      return fail(FR_ERR_CUDA, "begin capture");
+    }
+    const long long before = total_launches();
+    for (int i = 0; i < steps; i++) step_once(i == steps - 1);
+    graphKernels[steps] = (int)(total_launches() - before);
+    launches -= graphKernels[steps];  // counted again at every replay
+    iter = saveIter;
+    if (cudaStreamEndCapture(stream, &g) != cudaSuccess) return fail(FR_ERR_CUDA, "end capture");
+    const bool ok = cudaGraphInstantiate(&graphs[steps], g, 0) == cudaSuccess;
+    cudaGraphDestroy(g);
+    if (!ok) graphs[steps] = nullptr;
+    return ok || fail(FR_ERR_CUDA, "graph instantiate");
   }
 
   bool run(int n) {
@@ -1759,43 +1989,23 @@ struct fr_case {
     // the first iteration differs (wave-speed initialisation); run it eagerly
     while (n > 0 && iter < 1) {
       iter++;
-      if (!step_once()) return false;
+      if (!step_once(n == 1)) return false;
       n--;
     }
-    if (n <= 0) return true;
-    // the steady-state step (or kRunChunk of them) captured once
-    auto capture = [&](int steps, cudaGraphExec_t &exec, int &kernels) {
-      if (!stream) return fail(FR_ERR_STATE, "graph capture needs a non-default stream");
-      cudaGraph_t g;
-      long long saveIter = iter;
-      iter = 2;  // steady-state branch
-      if (cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
-        return fail(FR_ERR_CUDA, "begin capture");
-      long long before = total_launches();
-      for (int i = 0; i < steps; i++) step_once();
-      kernels = (int)(total_launches() - before);
-      launches -= kernels;  // counted again at every replay
-      if (cudaStreamEndCapture(stream, &g) != cudaSuccess) return fail(FR_ERR_CUDA, "end capture");
-      iter = saveIter;
-      if (cudaGraphInstantiate(&exec, g, 0) != cudaSuccess) {
-        cudaGraphDestroy(g);
-        return fail(FR_ERR_CUDA, "graph instantiate");
+    // the steady-state steps, captured once per number of steps
+    while (n > 0) {
+      const int k = std::min(n, kRunChunk);
+      if (!graphs[k] && !capture(k)) return false;
+      iter += k;
+      if (cudaGraphLaunch(graphs[k], stream) != cudaSuccess) return fail(FR_ERR_CUDA, "graph launch");
+      launches += graphKernels[k];
+      n -= k;
+      if (fused_ok()) {
+        fnStale = true;
+        fnOld = !(in.PMG && !levels.empty());
       }
-      cudaGraphDestroy(g);
-      return true;
-    };
-    if (n >= kRunChunk && !graphK && !capture(kRunChunk, graphK, graphKernelsK)) return false;
-    for (; n >= kRunChunk; n -= kRunChunk) {
-      iter += kRunChunk;
-      if (cudaGraphLaunch(graphK, stream) != cudaSuccess) return fail(FR_ERR_CUDA, "graph launch");
-      launches += graphKernelsK;
     }
-    if (n > 0 && !graph && !capture(1, graph, graphKernels)) return false;
-    for (int i = 0; i < n; i++) {
-      iter++;
-      if (cudaGraphLaunch(graph, stream) != cudaSuccess) return fail(FR_ERR_CUDA, "graph launch");
-      launches += graphKernels;
-    }
+    if (fnPinned) ensure_fn();
     return cuda_ok("run");
   }
 
@@ -2410,14 +2620,7 @@ int fr_get_info(fr_case *c, fr_info *info) {
 
 int fr_set_stream(fr_case *c, void *stream) {
   if (!c) return FR_ERR_ARG;
-  if (c->graph) {
-    cudaGraphExecDestroy(c->graph);
-    c->graph = nullptr;
-  }
-  if (c->graphK) {
-    cudaGraphExecDestroy(c->graphK);
-    c->graphK = nullptr;
-  }
+  c->drop_graphs();
   c->stream = (cudaStream_t)stream;
   // the coarse P-multigrid levels run on the case's stream too (left on the
   // old one, a captured step would miss their work)
@@ -2461,7 +2664,7 @@ int fr_set_state(fr_case *c, const double *U, size_t count) {
     return FR_ERR_CUDA;
   }
   if (c->mixed) c->split_state();
-  c->extrapolate();
+  c->renew_traces();
   if (c->in.dtType != 0)  // solver::initializeSolution, solver.cpp:1932-1938
     c->wavesp_init();
   c->stateSet = true;
@@ -2581,7 +2784,7 @@ int fr_calc_dt(fr_case *c, double *dtOut) {
   }
   long long save = c->iter;
   if (c->iter == 0) c->iter = 1;  // wave speeds from the current U_fpts
-  if (!c->fptsFresh) c->extrapolate();
+  if (!c->fptsFresh) c->renew_traces();
   c->calc_dt_dev();
   c->iter = save;
   if (!c->sync()) return FR_ERR_CUDA;
@@ -2678,7 +2881,10 @@ int fr_get_array(fr_case *c, const char *name, void *host, size_t *count) {
     if (n == "U_comp") return copy_dev(c, m.comp, nU, host, count);
     if (n == "U0") return copy_dev(c, m.U0, nU, host, count);
     if (n == "U_fpts") return copy_dev(c, m.Ufpts, nUf, host, count);
-    if (n == "Fn_fpts") return copy_dev(c, m.Fn, nUf, host, count);
+    if (n == "Fn_fpts") {
+      c->ensure_fn();
+      return copy_dev(c, m.Fn, nUf, host, count);
+    }
     if (n == "F_spts") return copy_dev(c, m.Fdbg, (size_t)c->nDims * nU, host, count);
     if (n == "disFn_fpts") return copy_dev(c, m.disFnDbg, nUf, host, count);
     if (n == "dUc_fpts") return copy_dev(c, m.dUc, nUf, host, count);
@@ -2693,7 +2899,10 @@ int fr_get_array(fr_case *c, const char *name, void *host, size_t *count) {
   if (n == "U_spts") return copy_dev(c, c->U, nU, host, count);
   if (n == "U0") return copy_dev(c, c->U0, nU, host, count);
   if (n == "U_fpts") return copy_dev(c, c->Ufpts, nUf, host, count);
-  if (n == "Fn_fpts") return copy_dev(c, c->Fn, nUf, host, count);
+  if (n == "Fn_fpts") {
+    c->ensure_fn();
+    return copy_dev(c, c->Fn, nUf, host, count);
+  }
   if (n == "waveSp_fpts") return copy_dev(c, c->waveSp, (size_t)c->nFp * c->E, host, count);
   if (n == "ele_dt") return copy_dev(c, c->eleDt, (size_t)c->E, host, count);
   if (n == "F_spts") return copy_dev(c, c->Fdbg, (size_t)c->nDims * nU, host, count);
@@ -2764,6 +2973,8 @@ int fr_device_ptr(fr_case *c, const char *name, void **ptr, size_t *bytes) {
       p = c->f32.Ufpts;
       b = nUf * 4;
     } else if (n == "Fn_fpts") {
+      c->fnPinned = true;
+      c->ensure_fn();
       p = c->f32.Fn;
       b = nUf * 4;
     } else if (n.rfind("divF_", 0) == 0) {
@@ -2785,6 +2996,8 @@ int fr_device_ptr(fr_case *c, const char *name, void **ptr, size_t *bytes) {
     p = c->Ufpts;
     b = nUf * 8;
   } else if (n == "Fn_fpts") {
+    c->fnPinned = true;
+    c->ensure_fn();
     p = c->Fn;
     b = nUf * 8;
   } else if (n.rfind("divF_", 0) == 0) {
@@ -2808,7 +3021,13 @@ int fr_bench_kernel(fr_case *c, const char *kernel, int reps) {
     return FR_ERR_STATE;
   }
   std::string k = kernel;
-  if (k == "faces") {
+  if (k == "stage") {
+    if (!c->fused_ok()) {
+      c->err = "this case's stages are two launches";
+      return FR_ERR_UNSUPPORTED;
+    }
+    for (int i = 0; i < reps; i++) c->fused_stage(1, false, false, false, false);
+  } else if (k == "faces") {
     for (int i = 0; i < reps; i++) c->faces_pass();
   } else if (k == "element_stage") {
     const int mode = c->in.timeType >= 5 ? frk::MODE_JAMESON : frk::MODE_RK_STAGE;
@@ -3045,7 +3264,7 @@ int fr_write_data(fr_case *c, const char *path) {
     size_t cnt = nU;
     int st = fr_get_array(c, "U_spts", U.data(), &cnt);
     if (st != FR_OK) return st;
-    if (!c->fptsFresh) c->extrapolate();
+    if (!c->fptsFresh) c->renew_traces();
     cnt = nUf;
     if ((st = fr_get_array(c, "U_fpts", Uf.data(), &cnt)) != FR_OK) return st;
     std::snprintf(name, sizeof name, ".csv.%.09lld", c->iter);

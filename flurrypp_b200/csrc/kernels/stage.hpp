@@ -231,6 +231,49 @@ void launch_element_stage_tma_visc(int nDims, int order, const ElemArgsT<R> &a, 
 template <typename R>
 void launch_elem_grad_tma(int nDims, int order, int E, const TpTablesT<R> &t, const TmaMaps &m,
                           unsigned int *err, cudaStream_t st);
+// One RK stage of an inviscid static case in one launch (stage_fused.cu):
+// every element forms the common flux of its own face points from its trace
+// and its neighbour's.  Metrics, normals and neighbour slots in thread order
+// (launch_fused_pack); the traces alternate between two buffers.
+enum FusedMode : int { FUSED_RESIDUAL = 0, FUSED_STAGE = 1, FUSED_FINAL = 2 };
+template <typename R>
+struct FusedArgsT {
+  int E = 0, mode = FUSED_RESIDUAL;
+  int first = 1;              // the input state is the step's base state
+  int loadS = 0, saveS = 0;   // the running sum of the passed stages is read / written
+  int keepU0 = 0;             // first stage: copy the base state to U0keep
+  double rka = 0.0, rkb = 0.0;
+  const R *Uin = nullptr, *Ufin = nullptr;
+  R *Uout = nullptr, *Ufout = nullptr, *U0keep = nullptr;
+  R *X0 = nullptr;            // the step's base state (thread order, written by the first stage)
+  R *S = nullptr;             // FP64: U0 - sum of RKb_s dt divF_s / detJ; FP32: without U0 (thread order)
+  R *comp = nullptr;          // FP32 final stage: rounding remainder of the state
+  R *divF = nullptr;          // optional: this stage's residual
+  const R *src = nullptr;     // P-multigrid source or null
+  const R *jg = nullptr, *rdet = nullptr, *nrm = nullptr;
+  const int *nb = nullptr;
+  const int *lineF = nullptr;  // [nDims][lines]: side-0 fpt | side-1 fpt << 16
+  const double *dt = nullptr, *eleDt = nullptr;
+  double *timeAcc = nullptr;   // final stage: *timeAcc += *dt
+  double *waveSp = nullptr;    // left-side wave speeds, or null
+  unsigned int *err = nullptr;
+  Phys ph{};
+  // the 1-D operators as kernel parameters (constant bank operands)
+  R D[36] = {}, E1[12] = {}, EFn1[12] = {}, C[12] = {};
+};
+struct FusedMaps {
+  CUtensorMap in, out, keep;  // [nS][E*nF]
+  CUtensorMap tr;             // [nFp][E*nF]
+};
+template <typename R>
+int fused_elems_per_block(int nDims, int order);
+// tma: the state rows allow TMA tiles (2-D always)
+template <typename R>
+void launch_fused_stage(int nDims, int order, bool tma, const FusedArgsT<R> &a, const FusedMaps &m, cudaStream_t st);
+// lineOf[f] = 2 * (dimension * lines + line) + side of every flux point
+template <typename R>
+void launch_fused_pack(int nDims, int order, int E, const R *JG, const R *det, const FaceTableT<R> &ft,
+                       const int *lineOf, R *jg, R *rdet, int *nb, R *nrm, cudaStream_t st);
 // Precision-form element stage on the tensor cores (tcgen05 kind::tf32,
 // 3xTF32) for 2-D orders 1..4 (32 elements per CTA) and 3-D order 1 (24);
 // the tile variant after the CUDA-core ones.  The operators are packed once

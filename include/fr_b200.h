@@ -63,7 +63,8 @@ typedef struct fr_setup_opts {
   int device;                  /* CUDA device ordinal; -1: host-side setup only */
   int generic_kernels;         /* 1: use the general sparse-operator element kernel */
   int no_tma;                  /* 1: tensor-product element kernel without TMA tiles */
-  int tile_variant;            /* precision form: element tile shape, -1 (default) = autotuned at setup;
+  int tile_variant;            /* -1 (default): one-launch stages where they apply; 0 and up: the two-kernel
+                                  form with that element tile shape (-1: autotuned at setup);
                                   the last variant of 2-D orders 1..4 is the tensor-core (tcgen05) kernel */
   int no_tensor_cores;         /* 1: leave the tensor-core variant out of the autotuner's choice */
   int no_pdl;                  /* 1: no programmatic dependent launch (used for small cases by default) */
@@ -245,8 +246,10 @@ int fr_read_restart(fr_case *c, const char *path);
 int fr_device_ptr(fr_case *c, const char *name, void **ptr, size_t *bytes);
 
 /* Instrumentation: launches one kernel of the steady-state RK stage `reps`
- * times on the case's stream ("element_stage": the fused element kernel of
- * an intermediate stage; "faces": the face kernel).  Mutates the state; for
+ * times on the case's stream ("stage": an intermediate stage in one launch,
+ * the form inviscid static cases run in, FR_ERR_UNSUPPORTED for others;
+ * "element_stage" and "faces": the element and face kernels of the two-kernel
+ * form).  Mutates the state; for
  * timing only.  No reference counterpart. */
 int fr_bench_kernel(fr_case *c, const char *kernel, int reps);
 
