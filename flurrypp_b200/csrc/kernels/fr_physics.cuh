@@ -163,16 +163,18 @@ template <typename R>
 __device__ __forceinline__ void roe2d(const R *UL, const R *UR, const R *n, R gamma, R *Fn) {
   const int nDims = 2;
   R vL[2], vR[2], um[2], du[4];
+  // one reciprocal per divisor instead of a division per term (18 of them)
+  const R rL = recip(UL[0]), rR = recip(UR[0]);
   for (int i = 0; i < nDims; i++) {
-    vL[i] = UL[i + 1] / UL[0];
-    vR[i] = UR[i + 1] / UR[0];
+    vL[i] = UL[i + 1] * rL;
+    vR[i] = UR[i + 1] * rR;
   }
   R pL = (gamma - R(1.0)) * (UL[3] - (R(0.5) * UL[0] * (vL[0] * vL[0] + vL[1] * vL[1])));
   R pR = (gamma - R(1.0)) * (UR[3] - (R(0.5) * UR[0] * (vR[0] * vR[0] + vR[1] * vR[1])));
-  R hL = (UL[nDims + 1] + pL) / UL[0];
-  R hR = (UR[nDims + 1] + pR) / UR[0];
-  R sq_rho = sqrt(UR[0] / UL[0]);
-  R rrho = R(1.) / (sq_rho + R(1.));
+  R hL = (UL[nDims + 1] + pL) * rL;
+  R hR = (UR[nDims + 1] + pR) * rR;
+  R sq_rho = root(UR[0] * rL);
+  R rrho = recip(sq_rho + R(1.));
   R usq = R(0.), unm = R(0.);
   for (int i = 0; i < nDims; i++) {
     um[i] = rrho * (vL[i] + sq_rho * vR[i]);
@@ -181,7 +183,7 @@ __device__ __forceinline__ void roe2d(const R *UL, const R *UR, const R *n, R ga
   }
   R hm = rrho * (hL + sq_rho * hR);
   R am_sq = (gamma - R(1.)) * (hm - usq);
-  R am = sqrt(am_sq);
+  R am = root(am_sq);
   R rhoUnL = R(0.), rhoUnR = R(0.);
   for (int i = 0; i < nDims; i++) {
     rhoUnL += UL[i + 1] * n[i];
@@ -195,14 +197,15 @@ __device__ __forceinline__ void roe2d(const R *UL, const R *UR, const R *n, R ga
   R lambda0 = fabs(unm);
   R lambdaP = fabs(unm + am);
   R lambdaM = fabs(unm - am);
-  R eps = R(0.5) * (fabs(rhoUnL / UL[0] - rhoUnR / UR[0]) +
-                    fabs(sqrt(gamma * pL / UL[0]) - sqrt(gamma * pR / UR[0])));
-  if (lambda0 < R(2.) * eps) lambda0 = R(0.25) * lambda0 * lambda0 / eps + eps;
-  if (lambdaP < R(2.) * eps) lambdaP = R(0.25) * lambdaP * lambdaP / eps + eps;
-  if (lambdaM < R(2.) * eps) lambdaM = R(0.25) * lambdaM * lambdaM / eps + eps;
+  R eps = R(0.5) * (fabs(rhoUnL * rL - rhoUnR * rR) + fabs(root(gamma * pL * rL) - root(gamma * pR * rR)));
+  const R re = recip(eps);  // unused where eps is 0
+  if (lambda0 < R(2.) * eps) lambda0 = R(0.25) * lambda0 * lambda0 * re + eps;
+  if (lambdaP < R(2.) * eps) lambdaP = R(0.25) * lambdaP * lambdaP * re + eps;
+  if (lambdaM < R(2.) * eps) lambdaM = R(0.25) * lambdaM * lambdaM * re + eps;
+  const R ra = recip(am);
   R a2 = R(0.5) * (lambdaP + lambdaM) - lambda0;
-  R a3 = R(0.5) * (lambdaP - lambdaM) / am;
-  R a1 = a2 * (gamma - R(1.)) / am_sq;
+  R a3 = R(0.5) * (lambdaP - lambdaM) * ra;
+  R a1 = a2 * (gamma - R(1.)) * (ra * ra);
   R a4 = a3 * (gamma - R(1.));
   R a5 = usq * du[0] - um[0] * du[1] - um[1] * du[2] + du[3];
   R a6 = unm * du[0] - n[0] * du[1] - n[1] * du[2];
