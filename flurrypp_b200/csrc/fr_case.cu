@@ -2816,25 +2816,23 @@ int fr_residual_norm(fr_case *c, int resType, double *out, int nFields) {
     return FR_ERR_STATE;
   }
   if (c->mixed)
-    frk::launch_residual_norm<float>(c->nS, c->E, c->nF, c->f32.divF[0], c->detJ, c->wSpt, resType, c->eleRes,
-                                     c->stream);
+    frk::launch_norm_total<float>(c->nS, c->E, c->nF, c->f32.divF[0], c->detJ, c->wSpt, resType, c->eleRes,
+                                  c->dtCount, c->stream);
   else
-    frk::launch_residual_norm<double>(c->nS, c->E, c->nF, c->divF[0], c->detJ, c->wSpt, resType, c->eleRes,
-                                      c->stream);
-  std::vector<double> er((size_t)c->E * c->nF);
+    frk::launch_norm_total<double>(c->nS, c->E, c->nF, c->divF[0], c->detJ, c->wSpt, resType, c->eleRes, c->dtCount,
+                                   c->stream);
+  double r[5];
   if (!c->sync()) return FR_ERR_CUDA;
-  cudaMemcpy(er.data(), c->eleRes, er.size() * sizeof(double), cudaMemcpyDeviceToHost);
+  if (cudaMemcpy(r, c->eleRes, c->nF * sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess) {
+    c->err = "residual norm read failed";
+    return FR_ERR_CUDA;
+  }
   for (int k = 0; k < c->nF; k++) {
-    double r = 0;
-    for (int e = 0; e < c->E; e++) {
-      double v = er[(size_t)e * c->nF + k];
-      if (v != v) {
-        c->err = "NaN Encountered in Solution Residual!";
-        return FR_ERR_NONFINITE;
-      }
-      r = resType == 3 ? std::max(r, v) : r + v;
+    if (r[k] != r[k]) {
+      c->err = "NaN Encountered in Solution Residual!";
+      return FR_ERR_NONFINITE;
     }
-    out[k] = resType == 2 ? std::sqrt(r) : r;
+    out[k] = resType == 2 ? std::sqrt(r[k]) : r[k];
   }
   return FR_OK;
 }

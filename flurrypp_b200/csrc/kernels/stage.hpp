@@ -348,6 +348,12 @@ template <typename R>
 void launch_residual_norm(int nS, int E, int nF, const R *divF, const double *detJ,
                           const double *wSpt, int resType, double *eleRes, cudaStream_t st);
 
+// The norm's total per field (before the root of resType 2) into
+// part[0 .. nF); part: E nF values of scratch, count: zero before and after.
+template <typename R>
+void launch_norm_total(int nS, int E, int nF, const R *divF, const double *detJ, const double *wSpt, int resType,
+                       double *part, unsigned int *count, cudaStream_t st);
+
 // Device health: counts non-finite or non-positive density entries in U.
 template <typename R>
 void launch_check_state(int nS, int E, int nF, const R *U, unsigned int *bad, cudaStream_t st);

@@ -602,6 +602,64 @@ __global__ void k_residual_norm(int nS, int E, int nF, const R *__restrict__ div
   }
 }
 
+// The whole norm's sums (or maxima) per field in one launch: a thread keeps
+// one field and walks the points with the grid's stride, so a warp reads
+// consecutive values; blocks leave partial values, and the last one to finish
+// folds them into part[0 .. nF) and resets the counter.  Against a thread per
+// element (stride nF, nS nF divisions in a chain, 115 CTAs at 14,637 hexes)
+// with every element's value copied to the host and added there: 3-D P3
+// 41x21x17, residual and norm, 388 -> 145 us.
+constexpr int kNormPts = 64;  // points of a block at a time
+template <typename R>
+__global__ void k_norm_total(int nF, long long nSE, int E, const R *__restrict__ divF, const double *__restrict__ detJ,
+                             const double *__restrict__ w, int resType, double *part, unsigned int *count) {
+  pdl_wait();
+  pdl_trigger();
+  extern __shared__ double sh[];  // [kNormPts][nF]
+  __shared__ bool last;
+  const int k = threadIdx.x % nF, j0 = threadIdx.x / nF;
+  const auto fold = [&](double v) {  // over the block's points, per field
+    sh[threadIdx.x] = v;
+    for (int o = kNormPts / 2; o > 0; o /= 2) {
+      __syncthreads();
+      if (j0 < o) {
+        const double b = sh[threadIdx.x + o * nF];
+        sh[threadIdx.x] = resType == 3 ? nan_max(sh[threadIdx.x], b) : sh[threadIdx.x] + b;
+      }
+    }
+  };
+  double r = 0;
+#pragma unroll 4
+  for (long long j = (long long)blockIdx.x * kNormPts + j0; j < nSE; j += (long long)gridDim.x * kNormPts) {
+    const double d = divF[j * nF + k];
+    if (resType == 1)
+      r += fabs(d) * w[(int)(j / E)];
+    else if (resType == 2)
+      r += d * d * recip(detJ[j]) * w[(int)(j / E)];
+    else  // a NaN anywhere makes the maximum NaN (fmax would drop it)
+      r = nan_max(fabs(d) * recip(detJ[j]), r);
+  }
+  fold(r);
+  if (j0 == 0) {
+    part[blockIdx.x * nF + k] = sh[k];
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(count, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  r = 0;
+  for (int b = j0; b < gridDim.x; b += kNormPts) {
+    const double v = __ldcg(&part[b * nF + k]);
+    r = resType == 3 ? nan_max(v, r) : r + v;
+  }
+  __syncthreads();
+  fold(r);
+  if (j0 == 0) part[k] = sh[k];
+  if (threadIdx.x == 0) *count = 0;
+}
+
 template <typename R>
 __global__ void k_add(long long n, R *__restrict__ out, const R *__restrict__ x, const R *__restrict__ y, double sgn) {
   pdl_wait();
@@ -788,6 +846,21 @@ void launch_residual_norm(int nS, int E, int nF, const R *divF, const double *de
   if (E <= 0) return;
   launch_k(k_residual_norm<R>, (E + 127) / 128, 128, 0, st, nS, E, nF, divF, detJ, wSpt, resType, eleRes);
 }
+
+template <typename R>
+void launch_norm_total(int nS, int E, int nF, const R *divF, const double *detJ, const double *wSpt, int resType,
+                       double *part, unsigned int *count, cudaStream_t st) {
+  const long long nSE = (long long)nS * E;
+  // at most one block per element: part holds E nF values
+  const long long want = (nSE + 4 * kNormPts - 1) / (4 * kNormPts);
+  const int grid = (int)std::min<long long>(std::min<long long>(want, E), 4LL * sm_count(current_device()));
+  launch_k(k_norm_total<R>, grid, kNormPts * nF, kNormPts * nF * sizeof(double), st, nF, nSE, E, divF, detJ, wSpt,
+           resType, part, count);
+}
+template void launch_norm_total<double>(int, int, int, const double *, const double *, const double *, int, double *,
+                                        unsigned int *, cudaStream_t);
+template void launch_norm_total<float>(int, int, int, const float *, const double *, const double *, int, double *,
+                                       unsigned int *, cudaStream_t);
 
 void launch_add(long long n, double *out, const double *x, const double *y, double sgn, cudaStream_t st) {
   if (n <= 0) return;
