@@ -195,7 +195,8 @@ struct fr_case {
     FusedDev<float> f;
   } fz;
   std::vector<double> hD, hE1, hEF, hLC;  // the 1-D operator tables (build_tp)
-  std::vector<int> hLineF, hLineOf;
+  std::vector<int> hLineF, hLineOf, hPairOf;
+  int *ldgNb = nullptr;  // FP32 3-D viscous: the neighbour table of the LDG jumps
   // Fn_fpts is formed on demand after one-launch stages, from the traces of
   // the last evaluation (fnOld: in the second trace buffer, else in U_fpts);
   // fnPinned: a caller holds its device pointer, so every call refreshes it
@@ -556,7 +557,7 @@ struct fr_case {
     } else if (useTp && !opts.no_tma && (E * nF) % 4 == 0) {
       if (!autotune_tiles()) return false;
     }
-    if (!setup_fused()) return false;
+    if (!setup_fused() || !setup_ldg()) return false;
     hostDt = in.dt;
     if (cudaMemcpyAsync(dt, &hostDt, sizeof(double), cudaMemcpyHostToDevice, stream) != cudaSuccess)
       return fail(FR_ERR_CUDA, "dt upload");
@@ -1030,6 +1031,8 @@ struct fr_case {
     const int nLines = nS / n;
     hLineF.assign((size_t)nDims * nLines, 0);
     hLineOf.assign(nFp, 0);
+    hPairOf.assign(nFp, 0);
+    for (size_t l = 0; l < pair.size(); l++) hPairOf[pair[l] & 0xffff] = 2 * l, hPairOf[pair[l] >> 16] = 2 * l + 1;
     for (int pr : pair) {
       const int f0 = pr & 0xffff, f1 = pr >> 16, d = fDn[f0], base = fBase[f0];
       const int c = d == nDims - 1 ? base : d == 0 ? base / n : base % n + base / (n * n) * n;
@@ -1240,6 +1243,26 @@ struct fr_case {
   bool build_tma(int v) {
     return build_maps<double>(tm, frk::tma_elems_per_block<double>(nDims, in.order, v), U, U0, acc, nullptr, Fn,
                               Ufpts, detJ, JGinv, detTma, jgTma, dUs, dUc, dUf);
+  }
+
+  // FP32 3-D viscous cases with TMA tiles form the LDG jumps in the gradient kernel
+  bool setup_ldg() {
+    if (!in.viscous || nDims != 3 || !mixed || !f32.useTma || (long long)nFp * E >= frk::kLdgPenBit) return true;
+    const int eb = frk::tma_elems_per_block<float>(nDims, in.order);
+    int *pairOf = nullptr;
+    if (!upload(pairOf, hPairOf) || !alloc(ldgNb, (size_t)((E + eb - 1) / eb) * eb * nFp)) return false;
+    frk::launch_ldg_pack(nDims, in.order, E, f32.ft, pairOf, ldgNb, stream);
+    return cuda_ok("LDG table");
+  }
+  // keep: store the jumps where a caller can see them (dUc_fpts)
+  frk::LdgArgsT<float> ldg_args(bool keep) {
+    frk::LdgArgsT<float> l;
+    l.nb = ldgNb;
+    l.Uf = f32.Ufpts;
+    l.dUc = f32.dUc;
+    l.keep = keep;
+    l.penFact = (float)ph.penFact;
+    return l;
   }
 
   // One-launch stages: inviscid static cases with tensor-product operators
@@ -1743,11 +1766,12 @@ struct fr_case {
   // (fixed dt per member) does not store them
   double *wave_out() { return perElementDt && in.dtType == 0 ? nullptr : waveSp; }
 
-  void faces_pass() {
+  // keepJumps: dUc_fpts of this evaluation can be looked at
+  void faces_pass(bool keepJumps = true) {
     const int nk = (ft.nInterior > 0 ? 1 : 0) + (ft.n > ft.nInterior ? 1 : 0);
     const int nkInv = (nk == 2 && frk::pdl_enabled()) ? 1 : nk;  // small cases: one face launch
     if (mixed) {
-      faces_pass32(nk);
+      faces_pass32(nk, keepJumps);
       return;
     }
     if (!in.viscous) {
@@ -1772,19 +1796,19 @@ struct fr_case {
     g.sStride = (long long)nS * E * nF;
     g.fStride = (long long)nFp * E * nF;
     if (useTma)
-      frk::launch_elem_grad_tma<double>(nDims, in.order, E, tp, tm, devErr, stream);
+      frk::launch_elem_grad_tma<double>(nDims, in.order, E, tp, tm, frk::LdgArgsT<double>{}, devErr, stream);
     else
       frk::launch_elem_grad(nDims, in.order, g, tp, stream);
     frk::launch_faces_visc(nDims, ft, Ufpts, dUf, g.fStride, Fn, wave_out(), ph, stream);
     launches += 2 * nk + 1;
   }
-  void faces_pass32(int nk) {
+  void faces_pass32(int nk, bool keepJumps) {
     if (!in.viscous) {
       frk::launch_faces_inviscid<float>(nDims, f32.ft, f32.Ufpts, f32.Fn, wave_out(), ph, stream);
       launches += (nk == 2 && frk::pdl_enabled()) ? 1 : nk;
       return;
     }
-    frk::launch_faces_ldg<float>(nDims, f32.ft, f32.Ufpts, f32.dUc, ph, stream);
+    frk::launch_faces_ldg<float>(nDims, f32.ft, f32.Ufpts, f32.dUc, ph, stream, ldgNb != nullptr);
     frk::GradArgsT<float> g;
     g.E = E;
     g.U = f32.U;
@@ -1795,12 +1819,12 @@ struct fr_case {
     g.dUf = f32.dUf;
     g.sStride = (long long)nS * E * nF;
     g.fStride = (long long)nFp * E * nF;
-    if (f32.useTma)
-      frk::launch_elem_grad_tma<float>(nDims, in.order, E, f32.tp, f32.tm, devErr, stream);
+    if (f32.useTma && (nDims == 2 || ldgNb))
+      frk::launch_elem_grad_tma<float>(nDims, in.order, E, f32.tp, f32.tm, ldg_args(keepJumps), devErr, stream);
     else
       frk::launch_elem_grad<float>(nDims, in.order, g, f32.tp, stream);
     frk::launch_faces_visc<float>(nDims, f32.ft, f32.Ufpts, f32.dUf, g.fStride, f32.Fn, wave_out(), ph, stream);
-    launches += 2 * nk + 1;
+    launches += 2 * nk + 1 - (ldgNb && ft.nInterior > 0 ? 1 : 0);
   }
   void element(const frk::ElemArgs &a) {
     if (in.viscous && useTma)
@@ -1924,11 +1948,11 @@ struct fr_case {
     const bool jameson = in.timeType >= 5;
     for (int step = 0; step < nRK - 1; step++) {
       if (step == 0 && in.dtType != 0) calc_dt_dev();
-      faces_pass();
+      faces_pass(false);
       element_stage(jameson ? frk::MODE_JAMESON : frk::MODE_RK_STAGE, step, in.RKa[step + 1],
                     jameson ? 0.0 : in.RKb[step], step == 0, pmgSource);
     }
-    faces_pass();
+    faces_pass(last && !pmgCoarse);
     if (nRK == 1 && in.dtType != 0) calc_dt_dev();
     if (jameson)
       element_stage(frk::MODE_JAMESON, nRK - 1, in.RKa[nRK], 0.0, nRK == 1, pmgSource);
@@ -3026,7 +3050,7 @@ int fr_bench_kernel(fr_case *c, const char *kernel, int reps) {
     }
     for (int i = 0; i < reps; i++) c->fused_stage(1, false, false, false, false);
   } else if (k == "faces") {
-    for (int i = 0; i < reps; i++) c->faces_pass();
+    for (int i = 0; i < reps; i++) c->faces_pass(false);
   } else if (k == "element_stage") {
     const int mode = c->in.timeType >= 5 ? frk::MODE_JAMESON : frk::MODE_RK_STAGE;
     const int stage = c->nRK > 1 ? 1 : 0;

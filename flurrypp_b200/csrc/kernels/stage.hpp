@@ -226,11 +226,27 @@ void launch_element_stage_tma(int nDims, int order, const ElemArgsT<R> &a, const
 template <typename R>
 void launch_element_stage_tma_visc(int nDims, int order, const ElemArgsT<R> &a, const TpTablesT<R> &t,
                                    const TmaMaps &m, cudaStream_t st);
+// What the FP32 3-D gradient kernel forms the LDG jumps from (the others read dUc):
+// nb[block][side][line, element] is the neighbour's slot with kLdgLeftBit where
+// this side is the face's left side and kLdgPenBit where the penalty changes
+// sign, or -(bc + 2), where the jump is in dUc already.
+constexpr int kLdgLeftBit = 1 << 30, kLdgPenBit = 1 << 29;
+template <typename R>
+struct LdgArgsT {
+  const int *nb = nullptr;
+  const R *Uf = nullptr;  // [nFp][E][nF]
+  R *dUc = nullptr;       // [nFp][E][nF] boundary jumps in; with keep, all of them out
+  int keep = 0;           // a caller can look at dUc after this evaluation
+  R penFact = R(0);
+};
 // Corrected physical gradient at the solution and flux points with TMA tiles
 // (U, dUc, JGinv, detJ in; dUs, dUf out), element block of tile variant 0.
 template <typename R>
 void launch_elem_grad_tma(int nDims, int order, int E, const TpTablesT<R> &t, const TmaMaps &m,
-                          unsigned int *err, cudaStream_t st);
+                          const LdgArgsT<R> &ldg, unsigned int *err, cudaStream_t st);
+// FP32 3-D: the neighbour table; pairOf[f] = 2 * (index of its line in linePair) + side.
+void launch_ldg_pack(int nDims, int order, int E, const FaceTableT<float> &ft, const int *pairOf, int *nb,
+                     cudaStream_t st);
 // One RK stage of an inviscid static case in one launch (stage_fused.cu):
 // every element forms the common flux of its own face points from its trace
 // and its neighbour's.  Metrics, normals and neighbour slots in thread order
@@ -306,7 +322,7 @@ struct GradArgsT {
 using GradArgs = GradArgsT<double>;
 template <typename R>
 void launch_faces_ldg(int nDims, const FaceTableT<R> &ft, const R *Ufpts, R *dUc, const Phys &ph,
-                      cudaStream_t st);
+                      cudaStream_t st, bool boundaryOnly = false);
 template <typename R>
 void launch_elem_grad(int nDims, int order, const GradArgsT<R> &g, const TpTablesT<R> &t, cudaStream_t st);
 template <typename R>

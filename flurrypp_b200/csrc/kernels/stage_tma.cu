@@ -795,11 +795,65 @@ struct Tg2 {
   static constexpr int O_IDX = O_CV + al(NCT);
   static constexpr int O_BAR = O_IDX + al((int)((NFP + NCT + NFP / 2) * 4 / sizeof(R)) + 1);
   static constexpr size_t SMEM = sizeof(R) * (size_t)(O_BAR + AL) + 128;
+  // the jumps formed in this kernel (below); CTAs per SM to cut its registers
+  // for, where they leave a thread at least 64
+  static constexpr bool LDG = GLP && sizeof(R) == 4;
+  static constexpr int WT = (NT + 31) / 32 * 32;
+  static constexpr int ctas(int c) { return c <= 1 || 65536 / (WT * c) >= 64 ? c : ctas(c - 1); }
+  static constexpr int MINB = ctas((int)((228 * 1024) / (SMEM + 1024)) < 16 ? (int)((228 * 1024) / (SMEM + 1024)) : 16);
   static_assert(SMEM <= kMaxSmem, "gradient tile set does not fit in shared memory");
 };
 
+// A trace's LDG jump UC - U in its place, from the neighbour's record (at a
+// boundary point the jump itself, which the boundary kernel stored); written
+// to dUc where a caller can see it.
+template <int ND, typename R>
+__device__ __forceinline__ void ldg_jump(R (&u)[ND + 2], const R *rec, int nb, const LdgArgsT<R> &a, long long slot) {
+  constexpr int NF = ND + 2;
+  const bool left = nb & kLdgLeftBit;
+  const R pen = (nb & kLdgPenBit) ? -a.penFact : a.penFact;
+#pragma unroll
+  for (int k = 0; k < NF; k++) {
+    const R o = rec[k], ul = left ? u[k] : o, ur = left ? o : u[k];
+    const R uc = R(0.5) * (ul + ur) - pen * (ul - ur);
+    u[k] = nb < 0 ? o : uc - u[k];
+  }
+  if (a.keep && nb >= 0)
+#pragma unroll
+    for (int k = 0; k < NF; k++) a.dUc[slot * NF + k] = u[k];
+}
+
+// The neighbour table of the jumps, by (block, side, line and element).
+template <typename R>
+__global__ void k_pack_ldg(int nd, int items, int EB, int E, int n, const int *__restrict__ pairOf,
+                           const int *__restrict__ slotL, const int *__restrict__ slotR, const R *__restrict__ nrm,
+                           int *__restrict__ nb) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int sL = slotL[i], sR = slotR[i];
+  const R *v = &nrm[(long long)i * nd];
+  // the penalty's sign follows the left normal (face.cpp:596-604)
+  const int pen = v[0] + v[1] + sqrt(R(2.)) * v[nd - 1] < 0 ? kLdgPenBit : 0;
+  const auto put = [&](int slot, int other) {
+    const int f = slot / E, e = slot - f * E;
+    nb[((long long)(e / EB) * 2 + (pairOf[f] & 1)) * items + (pairOf[f] >> 1) * EB + e % EB] = other;
+  };
+  put(sL, sR < 0 ? sR : sR | pen | kLdgLeftBit);
+  if (sR >= 0) put(sR, sL | pen);
+}
+
+// FP32 3-D (LDG): the jumps (face.cpp:188-202, 588-615) are formed here, per
+// line, from the line's own traces (its state is in registers; the sums are
+// those of the stored traces, bit for bit) and the neighbours' records, copied
+// by the thread that uses them; as a kernel of their own they were written and
+// read once more.  Two steps of Navier-Stokes, FP32: 40^3 P1 0.97 -> 0.90 ms,
+// 32^3 P2 1.47 -> 1.35, 26^3 P3 1.62 -> 1.54, 24^3 P4 2.17 -> 2.18, 16^3 P5
+// 1.48 -> 1.44.  In FP64 it raises the registers past two CTAs per SM or
+// spills (24^3 P4 4.03 -> 4.24 ms, 40^3 P1 1.73 -> 1.78, 26^3 P3 2.88 ->
+// 2.84), so FP64 keeps the jump kernel.
 template <int ND, int P, typename R>
-__global__ void __launch_bounds__(Tg2<ND, P, R>::NT) k_grad_tma(int E, TpTablesT<R> t, unsigned int *err,
+__global__ void __launch_bounds__(Tg2<ND, P, R>::NT, Tg2<ND, P, R>::LDG ? Tg2<ND, P, R>::MINB : 0) k_grad_tma(int E, TpTablesT<R> t, unsigned int *err,
+                                                                const __grid_constant__ LdgArgsT<R> ldg,
                                                                 const __grid_constant__ TmaMaps mp) {
   pdl_wait();
   pdl_trigger();
@@ -834,9 +888,10 @@ __global__ void __launch_bounds__(Tg2<ND, P, R>::NT) k_grad_tma(int E, TpTablesT
   }
   __syncthreads();
   if (tid == 0) {
-    mbar_arrive_expect_tx(&bar[0], sizeof(R) * (NS * ROW + NFP * ROW + ND * NS * EB * ND + NS * EB));
+    mbar_arrive_expect_tx(&bar[0],
+                          sizeof(R) * (NS * ROW + (T::LDG ? 0 : NFP * ROW) + ND * NS * EB * ND + NS * EB));
     tma_load_2d(sU, &mp.U, e0 * NF, 0, &bar[0]);
-    tma_load_2d(sC, &mp.dUc, e0 * NF, 0, &bar[0]);
+    if (!T::LDG) tma_load_2d(sC, &mp.dUc, e0 * NF, 0, &bar[0]);
     tma_load_3d(sJ, &mp.J, e0 * ND, 0, 0, &bar[0]);
     tma_load_2d(sDet, &mp.det, e0, 0, &bar[0]);
   }
@@ -851,7 +906,28 @@ __global__ void __launch_bounds__(Tg2<ND, P, R>::NT) k_grad_tma(int E, TpTablesT
     sCF[i] = t.corrFpt[i];
     sCV[i] = t.corrVal[i];
   }
+  constexpr int ITEMS = NFP / 2 * EB;  // (line, element) pairs
+  const int *nbp = ldg.nb + (long long)blockIdx.x * 2 * ITEMS;
+  if constexpr (T::LDG) {
+    for (int it = tid; it < ITEMS; it += NT) {
+      const int l = it / EB, fe = it - (it / EB) * EB;
+      const int pr = t.linePair[l];
+#pragma unroll
+      for (int j = 0; j < 2; j++) {
+        const int nb = __ldg(nbp + j * ITEMS + it);
+        const int f = j ? pr >> 16 : pr & 0xffff;
+        if (fe < nValid) {
+          const R *src = nb >= 0 ? &ldg.Uf[(long long)(nb & (kLdgPenBit - 1)) * NF]
+                                 : &ldg.dUc[((long long)f * E + e0 + fe) * NF];
+#pragma unroll
+          for (int k = 0; k < NF; k++) cp_async_word(&sC[f * ROW + fe * NF + k], src + k);
+        }
+      }
+    }
+    cp_async_commit();
+  }
   const bool ok = __syncthreads_and(mbar_wait_bounded(&bar[0], 0, 1u << 22));
+  if constexpr (T::LDG) cp_async_wait<0>();  // this thread's neighbour records
   if (!ok) {
     if (tid == 0 && err) atomicOr(err, 1);
     mbar_wait_bounded(&bar[0], 0, 1u << 22);
@@ -887,10 +963,29 @@ __global__ void __launch_bounds__(Tg2<ND, P, R>::NT) k_grad_tma(int E, TpTablesT
       for (int m = 0; m < N; m++)
 #pragma unroll
         for (int k = 0; k < NF; k++) x[m][k] = sU[(base + m * stride) * ROW + fe * NF + k];
+      if constexpr (T::LDG) {
 #pragma unroll
-      for (int k = 0; k < NF; k++) {
-        q0[k] = sC[f0 * ROW + fe * NF + k];
-        q1[k] = sC[f1 * ROW + fe * NF + k];
+        for (int k = 0; k < NF; k++) q0[k] = q1[k] = R(0);
+#pragma unroll
+        for (int m = 0; m < N; m++) {
+          const R v0 = sE[m], v1 = sE[N + m];
+#pragma unroll
+          for (int k = 0; k < NF; k++) {
+            q0[k] += v0 * x[m][k];
+            q1[k] += v1 * x[m][k];
+          }
+        }
+        if (fe < nValid) {
+          const long long s0 = (long long)f0 * E + e0 + fe, s1 = (long long)f1 * E + e0 + fe;
+          ldg_jump<ND, R>(q0, &sC[f0 * ROW + fe * NF], __ldg(nbp + it), ldg, s0);
+          ldg_jump<ND, R>(q1, &sC[f1 * ROW + fe * NF], __ldg(nbp + ITEMS + it), ldg, s1);
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < NF; k++) {
+          q0[k] = sC[f0 * ROW + fe * NF + k];
+          q1[k] = sC[f1 * ROW + fe * NF + k];
+        }
       }
 #pragma unroll
       for (int i = 0; i < N; i++) {
@@ -1010,11 +1105,12 @@ __global__ void __launch_bounds__(Tg2<ND, P, R>::NT) k_grad_tma(int E, TpTablesT
 }
 
 template <int ND, int P, typename R>
-void launch_grad(int E, const TpTablesT<R> &t, const TmaMaps &m, unsigned int *err, cudaStream_t st) {
+void launch_grad(int E, const TpTablesT<R> &t, const TmaMaps &m, const LdgArgsT<R> &ldg, unsigned int *err,
+                 cudaStream_t st) {
   using T = Tg2<ND, P, R>;
   static std::atomic<unsigned long long> attrDev{0};
   smem_attr(k_grad_tma<ND, P, R>, (int)T::SMEM, attrDev);
-  launch_k(k_grad_tma<ND, P, R>, (E + T::EB - 1) / T::EB, T::NT, T::SMEM, st, E, t, err, m);
+  launch_k(k_grad_tma<ND, P, R>, (E + T::EB - 1) / T::EB, T::NT, T::SMEM, st, E, t, err, ldg, m);
 }
 
 template <typename R>
@@ -1040,18 +1136,18 @@ template void launch_element_stage_tma_visc<float>(int, int, const ElemArgsT<flo
                                                    const TmaMaps &, cudaStream_t);
 
 template <typename R>
-void launch_elem_grad_tma(int nDims, int order, int E, const TpTablesT<R> &t, const TmaMaps &m, unsigned int *err,
-                          cudaStream_t st) {
+void launch_elem_grad_tma(int nDims, int order, int E, const TpTablesT<R> &t, const TmaMaps &m,
+                          const LdgArgsT<R> &ldg, unsigned int *err, cudaStream_t st) {
   if (E <= 0) return;
 #define FR_TG_CASE(ND, P) \
-  if (nDims == ND && order == P) return launch_grad<ND, P, R>(E, t, m, err, st);
+  if (nDims == ND && order == P) return launch_grad<ND, P, R>(E, t, m, ldg, err, st);
   FR_TM_ORDERS(FR_TG_CASE)
 #undef FR_TG_CASE
 }
-template void launch_elem_grad_tma<double>(int, int, int, const TpTablesT<double> &, const TmaMaps &, unsigned int *,
-                                           cudaStream_t);
-template void launch_elem_grad_tma<float>(int, int, int, const TpTablesT<float> &, const TmaMaps &, unsigned int *,
-                                          cudaStream_t);
+template void launch_elem_grad_tma<double>(int, int, int, const TpTablesT<double> &, const TmaMaps &,
+                                           const LdgArgsT<double> &, unsigned int *, cudaStream_t);
+template void launch_elem_grad_tma<float>(int, int, int, const TpTablesT<float> &, const TmaMaps &,
+                                           const LdgArgsT<float> &, unsigned int *, cudaStream_t);
 
 int tma_variants(bool fp32) { return fp32 ? kFp32Variants : kFp64Variants; }
 
@@ -1092,6 +1188,14 @@ void launch_element_stage_tma<float>(int nDims, int order, const ElemArgsT<float
     launch_v<float, 1>(nDims, order, a, t, m, st);
   else
     launch_v<float, 2>(nDims, order, a, t, m, st);
+}
+
+void launch_ldg_pack(int nDims, int order, int E, const FaceTableT<float> &ft, const int *pairOf, int *nb,
+                     cudaStream_t st) {
+  const int N = order + 1, EB = tma_elems_per_block<float>(nDims, order, 0);
+  if (ft.n > 0)
+    k_pack_ldg<float><<<(ft.n + 255) / 256, 256, 0, st>>>(nDims, nDims * N * N * EB, EB, E, ft.n, pairOf, ft.slotL,
+                                                      ft.slotR, ft.nrm, nb);
 }
 
 }  // namespace frk

@@ -372,9 +372,9 @@ void launch_grad(const GradArgsT<R> &g, const TpTablesT<R> &t, cudaStream_t st) 
 }  // namespace
 
 template <typename R>
-void launch_faces_ldg(int nDims, const FaceTableT<R> &ft, const R *Ufpts, R *dUc, const Phys &ph, cudaStream_t st) {
+void launch_faces_ldg(int nDims, const FaceTableT<R> &ft, const R *Ufpts, R *dUc, const Phys &ph, cudaStream_t st, bool boundaryOnly) {
   const int b = 256, nI = ft.nInterior, nB = ft.n - ft.nInterior;
-  if (nI > 0) {
+  if (nI > 0 && !boundaryOnly) {
     const long long nt = (long long)nI * (nDims + 2);
     const unsigned g = (unsigned)((nt + b - 1) / b);
     if (nDims == 2)
@@ -423,7 +423,7 @@ void launch_elem_grad(int nDims, int order, const GradArgsT<R> &g, const TpTable
 }
 
 #define FR_VISC_INST(R)                                                                                    \
-  template void launch_faces_ldg<R>(int, const FaceTableT<R> &, const R *, R *, const Phys &, cudaStream_t);      \
+  template void launch_faces_ldg<R>(int, const FaceTableT<R> &, const R *, R *, const Phys &, cudaStream_t, bool); \
   template void launch_faces_visc<R>(int, const FaceTableT<R> &, const R *, const R *, long long, R *, double *, \
                                      const Phys &, cudaStream_t);                                                \
   template void launch_elem_grad<R>(int, int, const GradArgsT<R> &, const TpTablesT<R> &, cudaStream_t);
