@@ -29,9 +29,9 @@
 // and elements as two launches 0.063 + 0.170 ms), the rest the latency of its
 // barrier-separated phases at 18 warps per SM (96 registers); FP32 0.117 ms
 // (0.035 + 0.101 ms), 450 MB.  Four steps, two launches a stage -> one:
-// 3-D P3 32^3 3.71 -> 3.01 ms, FP32 2.16 -> 1.85; 3-D P2 27^3 (rows without
-// TMA) 1.89 -> 1.06; 2-D P3 256^2 1.05 -> 0.91, FP32 0.58 -> 0.42; 2-D P2
-// 384^2 FP32 0.81 -> 0.66; 20 steps of 2-D P3 32^2 206 -> 161 us.
+// 3-D P3 32^3 3.71 -> 2.98 ms, FP32 2.16 -> 1.85; 3-D P2 27^3 (rows without
+// TMA) 1.89 -> 1.02; 2-D P3 256^2 1.05 -> 0.91, FP32 0.58 -> 0.43; 2-D P2
+// 384^2 FP32 0.81 -> 0.66; 20 steps of 2-D P3 32^2 206 -> 160 us.
 // Tried and slower: one thread per line of one dimension only, working on all
 // three (half the threads: 3.33 ms at 32^3, 236 us at 32^2); element counts
 // of half or twice the ones below; starting the next wave's tiles for L2 ahead
@@ -260,26 +260,47 @@ __device__ __forceinline__ void end_flux(const R (&own)[ND + 2], const R *sNb, i
 }
 
 // Traces at both ends of a line of a dense tile (the state), N records apart
-// by `step`.  An x-line's records start a multiple of 128 bytes apart in 3-D,
-// so every lane starts at its own point (rot) and wraps round, which spreads
-// a warp over the banks; the order of the sum depends on the line only, so a
-// trace has the same bits here and where the last stage stored it.
-template <int N, int NF, typename R>
+// by `step`, summed in ascending order as everywhere.  ROT (3-D P3): the
+// x-lines' records start a multiple of 128 bytes apart, four deep on the same
+// banks, so a lane reads them from its own point on (rot), which spreads the
+// warp over the banks, and turns them back in registers.
+template <int N, int NF, bool ROT, typename R>
 __device__ __forceinline__ void line_ends(const R *base, int step, int rot, const R *sE, R (&t)[2][NF]) {
+  R x[N][NF];
+  if constexpr (ROT) {
+    static_assert(N == 4, "two conditional turns");
+    int m = rot;
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      lds<NF, R>(base + m * step, x[i]);
+      m = (m + 1) & 3;
+    }
+    if (rot != 0) {  // x[i] holds point (i + rot) % 4
+#pragma unroll
+      for (int k = 0; k < NF; k++) {
+        const R a = x[0][k], b = x[1][k], c = x[2][k], d = x[3][k];
+        const bool r1 = rot & 1, r2 = rot & 2;
+        const R e = r1 ? d : a, f = r1 ? a : b, g = r1 ? b : c, h = r1 ? c : d;
+        x[0][k] = r2 ? g : e;
+        x[1][k] = r2 ? h : f;
+        x[2][k] = r2 ? e : g;
+        x[3][k] = r2 ? f : h;
+      }
+    }
+  } else {
+#pragma unroll
+    for (int m = 0; m < N; m++) lds<NF, R>(base + m * step, x[m]);
+  }
 #pragma unroll
   for (int k = 0; k < NF; k++) t[0][k] = t[1][k] = R(0);
-  int m = rot;
 #pragma unroll
-  for (int i = 0; i < N; i++) {
-    R x[NF];
-    lds<NF, R>(base + m * step, x);
+  for (int m = 0; m < N; m++) {
     const R e0 = sE[m], e1 = sE[N + m];
 #pragma unroll
     for (int k = 0; k < NF; k++) {
-      t[0][k] += e0 * x[k];
-      t[1][k] += e1 * x[k];
+      t[0][k] += e0 * x[m][k];
+      t[1][k] += e1 * x[m][k];
     }
-    m = m + 1 == N ? 0 : m + 1;
   }
 }
 
@@ -323,12 +344,12 @@ __global__ void __launch_bounds__(Fz<ND, P, R>::NT, Fz<ND, P, R>::MINB)
   constexpr int N = T::N, NF = T::NF, NS = T::NS, NC = T::NC, NFP = T::NFP, EB = T::EB, NT = T::NT, ROW = T::ROW;
   constexpr int NPT = T::NPT, XROW = T::XROW;
   constexpr int PT = (NPT + NT - 1) / NT;  // points per thread
-  // the correction is added line by line, per direction; in 2-D FP64 at the
+  // the correction is added line by line, per direction, in 3-D; in 2-D at the
   // points, after the directions' sum and in the reference's face order, which
-  // makes its steps bit-identical to the two-kernel form's (one or two per
-  // cent slower; a run beyond its stability limit amplifies a last bit to
-  // 1e-11 in 20 steps)
-  constexpr bool CORR = ND == 3 || F32;
+  // makes the steps bit-identical to the two-kernel form's (20 steps of 32^2
+  // P3 FP64 145 -> 160 us; FP32 384^2 P2 653 -> 663 us, 256^2 P3 414 -> 431; a
+  // run beyond its stability limit amplifies a last bit to 1e-11 in 20 steps)
+  constexpr bool CORR = ND == 3;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   R *smem = reinterpret_cast<R *>(smem_align128(smem_raw));
   R *sU = smem + T::O_U, *sX = smem + T::O_X, *sY = smem + T::O_Y, *sQ = smem + T::O_Q, *sE = smem + T::O_E;
@@ -414,10 +435,11 @@ __global__ void __launch_bounds__(Fz<ND, P, R>::NT, Fz<ND, P, R>::MINB)
   // neighbours' records
   const int base = dim == ND - 1 ? col : dim == 0 ? col * N : col % N + col / N * (N * N);
   const int stride = dim == ND - 1 ? NC : dim == 0 ? 1 : N;
-  const int rot = (ND == 3 && dim == 0) ? col % N : 0;
+  constexpr bool ROT = ND == 3 && P == 3;
+  const int rot = (ROT && dim == 0) ? col % N : 0;
   {
     R t[2][NF], f0[NF], f1[NF];
-    line_ends<N, NF, R>(&sU[base * ROW + el * NF], stride * ROW, rot, sE, t);
+    line_ends<N, NF, ROT, R>(&sU[base * ROW + el * NF], stride * ROW, rot, sE, t);
     cp_async_wait<0>();  // this thread's neighbour records
     double *w0 = nullptr, *w1 = nullptr;
     if (a.waveSp && valid) {
@@ -617,7 +639,7 @@ __global__ void __launch_bounds__(Fz<ND, P, R>::NT, Fz<ND, P, R>::MINB)
   }
   {
     R t[2][NF];
-    line_ends<N, NF, R>(&sU[base * ROW + el * NF], stride * ROW, rot, sE, t);
+    line_ends<N, NF, ROT, R>(&sU[base * ROW + el * NF], stride * ROW, rot, sE, t);
     sts<NF, R>(q0, t[0]);
     sts<NF, R>(q1, t[1]);
   }
