@@ -557,7 +557,7 @@ struct fr_case {
     } else if (useTp && !opts.no_tma && (E * nF) % 4 == 0) {
       if (!autotune_tiles()) return false;
     }
-    if (!setup_fused() || !setup_ldg()) return false;
+    if (!setup_ldg()) return false;
     hostDt = in.dt;
     if (cudaMemcpyAsync(dt, &hostDt, sizeof(double), cudaMemcpyHostToDevice, stream) != cudaSuccess)
       return fail(FR_ERR_CUDA, "dt upload");
@@ -568,6 +568,7 @@ struct fr_case {
       if (!make_csr(op.prolong, op.nSptsPro, nS, prolongOp)) return false;
       if (!pmgCoarse && !build_levels()) return false;
     }
+    if (!setup_fused()) return false;  // last: it does without where memory is short
     if (cudaStreamSynchronize(stream) != cudaSuccess) return fail(FR_ERR_CUDA, "setup sync");
     return cuda_ok("setup");
   }
@@ -1283,7 +1284,6 @@ struct fr_case {
                                                   f32.detJ, f32.ft)
                           : setup_fused_as<double>(fz.d, lanes, eb, U, acc, U0, Ufpts, JGinv, detJ, ft);
     if (!ok) return false;
-    fz.on = true;
     return cuda_ok("one-launch stage setup");
   }
   template <typename R>
@@ -1301,6 +1301,12 @@ struct fr_case {
     const size_t oJ = take(lanes * n * nDims * nDims), oR = take(lanes * n), oN = take(lanes * 2 * nDims * (nDims + 1)),
                  oX = take(lanes * n * nF), oS = take(lanes * n * nF), oT = take(nUf),
                  oB = take((lanes * 2 * nDims * sizeof(int) + sizeof(R) - 1) / sizeof(R));
+    // a case that fills the memory keeps the two-kernel form
+    size_t freeBytes = 0, allBytes = 0;
+    if (cudaMemGetInfo(&freeBytes, &allBytes) != cudaSuccess || total * sizeof(R) > freeBytes / 2) {
+      cudaGetLastError();
+      return true;
+    }
     R *pool = nullptr;
     if (!alloc(pool, total)) return false;
     z.jg = pool + oJ, z.rdet = pool + oR, z.nrm = pool + oN, z.X0 = pool + oX, z.S = pool + oS, z.Uf2 = pool + oT;
@@ -1334,6 +1340,7 @@ struct fr_case {
     a.ph = ph;
     for (int i = 0; i < n * n; i++) a.D[i] = (R)hD[i];
     for (int i = 0; i < 2 * n; i++) a.E1[i] = (R)hE1[i], a.EFn1[i] = (R)hEF[i], a.C[i] = (R)hLC[i];
+    fz.on = true;
     return true;
   }
   bool fused_ok() const { return fz.on && cut.n == 0; }
