@@ -63,7 +63,7 @@ WORKLOAD = "3D Euler Taylor-Green vortex, 32^3 hexes, P=3, RK4, Rusanov, FP64 pl
 
 def profiled_traffic(kernel_tag: str):
     """DRAM bytes per launch of a kernel from the committed ncu summary."""
-    p = os.path.join(ROOT, "profiles", "fp64_stage_tgv32_p3.md")
+    p = os.path.join(ROOT, "profiles", "one_launch_stage.md")
     try:
         for line in open(p):
             if line.startswith(kernel_tag + ":"):
@@ -271,14 +271,6 @@ def state_errors(U, ref):
     per = [float(np.linalg.norm(d[..., k]) / max(np.linalg.norm(ref[..., k]), 1e-300)) for k in range(ref.shape[-1])]
     return {"l2_rel": float(np.linalg.norm(d) / np.linalg.norm(ref)),
             "max_rel": float(np.abs(d).max() / np.abs(ref).max()), "l2_rel_per_field": per}
-
-
-def elem_bytes(s, wbytes):
-    """Algorithmic bytes of one intermediate-stage element launch: read U, U0,
-    acc (3 nS nF), Fn (nFp nF), JGinv (nDims^2 nS), detJ (nS); write acc, U
-    (2 nS nF) and U_fpts (nFp nF); words of the working precision."""
-    nS, nFp, nF, nd, E = s.nSpts, s.nFpts, s.nFields, s.nDims, s.nEles
-    return wbytes * E * (5 * nS * nF + 2 * nFp * nF + nd * nd * nS + nS)
 
 
 def stage_bytes(s, wbytes):
@@ -995,7 +987,7 @@ def main():
             "gpu_launches": launches,
             "roofline": {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
                          "traffic": profiled_traffic("one_launch_traffic_bytes"),
-                         "traffic_source": "profiles/fp64_stage_tgv32_p3.md (ncu, one launch)",
+                         "traffic_source": "profiles/one_launch_stage.md (ncu, one launch)",
                          "kernel": "k_fused_stage<3, 3, double>",
                          "tile_variant": inf.tile_variant, "elems_per_block": inf.elems_per_block,
                          "kernel_ms": kt["stage"], "algorithmic_bytes": alg_bytes,
