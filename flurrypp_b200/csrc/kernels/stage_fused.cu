@@ -307,7 +307,10 @@ __device__ __forceinline__ void line_ends(const R *base, int step, int rot, cons
 // Along a line with flux values x: q comes in as the end fluxes and leaves as
 // the end jumps (flux minus extrapolated flux); y is the divergence, with
 // CORR plus the correction from both ends.  Every sum starts from zero, as in
-// the other element kernels, for the same contractions.
+// the other element kernels, for the same contractions; the FP32 correction's
+// contraction is written out, as the compiler forms it in k_elem_tma's line
+// pass (started from zero it rounds the other product: 1 to 17 % of the FP32
+// residuals moved by a last bit, and their FP64 norm by up to 4e-9).
 template <int N, int NF, bool CORR, typename R>
 __device__ __forceinline__ void line_div(const FusedArgsT<R> &a, const R (&x)[N][NF], R (&q)[2][NF], R (&y)[N][NF]) {
 #pragma unroll
@@ -327,8 +330,12 @@ __device__ __forceinline__ void line_div(const FusedArgsT<R> &a, const R (&x)[N]
 #pragma unroll
       for (int m = 0; m < N; m++) acc += a.D[i * N + m] * x[m][k];
       if constexpr (CORR) {
-        c += a.C[i] * q[0][k];
-        c += a.C[N + i] * q[1][k];
+        if constexpr (sizeof(R) == 4) {
+          c = fmaf(a.C[i], q[0][k], __fmul_rn(a.C[N + i], q[1][k]));
+        } else {
+          c += a.C[i] * q[0][k];
+          c += a.C[N + i] * q[1][k];
+        }
         y[i][k] = c + acc;
       } else {
         y[i][k] = acc;
@@ -344,12 +351,15 @@ __global__ void __launch_bounds__(Fz<ND, P, R>::NT, Fz<ND, P, R>::MINB)
   constexpr int N = T::N, NF = T::NF, NS = T::NS, NC = T::NC, NFP = T::NFP, EB = T::EB, NT = T::NT, ROW = T::ROW;
   constexpr int NPT = T::NPT, XROW = T::XROW;
   constexpr int PT = (NPT + NT - 1) / NT;  // points per thread
-  // the correction is added line by line, per direction, in 3-D; in 2-D at the
-  // points, after the directions' sum and in the reference's face order, which
-  // makes the steps bit-identical to the two-kernel form's (20 steps of 32^2
-  // P3 FP64 145 -> 160 us; FP32 384^2 P2 653 -> 663 us, 256^2 P3 414 -> 431; a
-  // run beyond its stability limit amplifies a last bit to 1e-11 in 20 steps)
-  constexpr bool CORR = ND == 3;
+  // where the correction is added: line by line, per direction, in 3-D FP64
+  // and in 3-D FP32 with TMA rows, as k_elem_tma does; at the points, after the
+  // directions' sum and in the reference's face order, in 2-D and in 3-D FP32
+  // without TMA rows, as k_elem_tp does.  This makes 2-D and FP32 steps
+  // bit-identical to the two-kernel form's (20 steps of 32^2 P3 FP64 145 -> 160
+  // us; FP32 384^2 P2 653 -> 663 us, 256^2 P3 414 -> 431; a run beyond its
+  // stability limit amplifies a last bit to 1e-11 in 20 steps); FP64 3-D differs
+  // in last bits (both its two-kernel forms add at the points)
+  constexpr bool CORR = ND == 3 && (!F32 || TMA);
   extern __shared__ __align__(128) unsigned char smem_raw[];
   R *smem = reinterpret_cast<R *>(smem_align128(smem_raw));
   R *sU = smem + T::O_U, *sX = smem + T::O_X, *sY = smem + T::O_Y, *sQ = smem + T::O_Q, *sE = smem + T::O_E;
@@ -555,14 +565,26 @@ __global__ void __launch_bounds__(Fz<ND, P, R>::NT, Fz<ND, P, R>::MINB)
 #pragma unroll
     for (int k = 0; k < NF; k++) div[i][k] += s1[k];
     if constexpr (!CORR) {
-      const int x = p % N, y = p / N, fx = __ldg(&a.lineF[y]), fy = __ldg(&a.lineF[NC + x]);
-      const int f[4] = {fy & 0xffff, fx >> 16, fy >> 16, fx & 0xffff};  // bottom, right, top, left
-      const R c[4] = {sE[2 * N + y], sE[3 * N + x], sE[3 * N + y], sE[2 * N + x]};
+      const int x = p % N, y = p / N % N, z = p / (N * N);
+      int f[2 * ND];
+      R c[2 * ND];
+      const R *c0 = sE + 2 * N, *c1 = sE + 3 * N;  // the correction of the two sides along a line
+      if constexpr (ND == 2) {
+        const int fx = __ldg(&a.lineF[y]), fy = __ldg(&a.lineF[NC + x]);
+        f[0] = fy & 0xffff, f[1] = fx >> 16, f[2] = fy >> 16, f[3] = fx & 0xffff;  // bottom, right, top, left
+        c[0] = c0[y], c[1] = c1[x], c[2] = c1[y], c[3] = c0[x];
+      } else {  // bottom, top, left, right, front, back
+        const int fz = __ldg(&a.lineF[2 * NC + x + N * y]), fx = __ldg(&a.lineF[y + N * z]),
+                  fy = __ldg(&a.lineF[NC + x + N * z]);
+        f[0] = fz & 0xffff, f[1] = fz >> 16, f[2] = fx & 0xffff, f[3] = fx >> 16;
+        f[2 * ND - 2] = fy & 0xffff, f[2 * ND - 1] = fy >> 16;
+        c[0] = c0[z], c[1] = c1[z], c[2] = c0[x], c[3] = c1[x], c[2 * ND - 2] = c0[y], c[2 * ND - 1] = c1[y];
+      }
       R cq[NF];
 #pragma unroll
       for (int k = 0; k < NF; k++) cq[k] = R(0);
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
+      for (int j = 0; j < 2 * ND; j++) {
         R q[NF];
         lds<NF, R>(&sQ[f[j] * ROW + o], q);
 #pragma unroll
