@@ -1996,22 +1996,42 @@ struct fr_case {
   bool capture(int steps) {
     if (!stream) return fail(FR_ERR_STATE, "graph capture needs a non-default stream");
     cudaGraph_t g;
-    const long long saveIter = iter;
-    iter = 2;  // steady-state branch
-    if (cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-      iter = saveIter;
+    if (cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
       return fail(FR_ERR_CUDA, "begin capture");
-    }
+    // nothing runs yet: what the steps leave is noted at each launch (replay)
+    const long long saveIter = iter;
+    const bool saveFresh = fptsFresh, saveStale = fnStale, saveOld = fnOld;
+    iter = 2;  // steady-state branch
     const long long before = total_launches();
     for (int i = 0; i < steps; i++) step_once(i == steps - 1);
     graphKernels[steps] = (int)(total_launches() - before);
     launches -= graphKernels[steps];  // counted again at every replay
     iter = saveIter;
+    fptsFresh = saveFresh, fnStale = saveStale, fnOld = saveOld;
     if (cudaStreamEndCapture(stream, &g) != cudaSuccess) return fail(FR_ERR_CUDA, "end capture");
     const bool ok = cudaGraphInstantiate(&graphs[steps], g, 0) == cudaSuccess;
     cudaGraphDestroy(g);
     if (!ok) graphs[steps] = nullptr;
     return ok || fail(FR_ERR_CUDA, "graph instantiate");
+  }
+
+  // `steps` steady-state steps as one graph launch.  A graph starts from
+  // traces of the current state, renewed here where they are stale, and never
+  // renews them itself, so it can be captured at any moment; a P-multigrid
+  // cycle leaves them stale (it prolongs into U).
+  bool replay(int steps) {
+    if (!fptsFresh && !mo.on) extrapolate();
+    if (!graphs[steps] && !capture(steps)) return false;
+    iter += steps;
+    if (cudaGraphLaunch(graphs[steps], stream) != cudaSuccess) return fail(FR_ERR_CUDA, "graph launch");
+    launches += graphKernels[steps];
+    const bool cycle = in.PMG && !levels.empty();
+    fptsFresh = !mo.on && !cycle;
+    if (fused_ok()) {
+      fnStale = true;
+      fnOld = !cycle;
+    }
+    return true;
   }
 
   bool run(int n) {
@@ -2023,19 +2043,9 @@ struct fr_case {
       if (!step_once(n == 1)) return false;
       n--;
     }
-    // the steady-state steps, captured once per number of steps
-    while (n > 0) {
-      const int k = std::min(n, kRunChunk);
-      if (!graphs[k] && !capture(k)) return false;
-      iter += k;
-      if (cudaGraphLaunch(graphs[k], stream) != cudaSuccess) return fail(FR_ERR_CUDA, "graph launch");
-      launches += graphKernels[k];
-      n -= k;
-      if (fused_ok()) {
-        fnStale = true;
-        fnOld = !(in.PMG && !levels.empty());
-      }
-    }
+    for (; n >= kRunChunk; n -= kRunChunk)
+      if (!replay(kRunChunk)) return false;
+    if (n > 0 && !replay(n)) return false;
     if (fnPinned) ensure_fn();
     return cuda_ok("run");
   }
