@@ -24,6 +24,8 @@ SEQUENCES = {
     "new state": [("run", 10), ("state", 1.01), ("run", 5), ("run", 5), ("run", 5)],
     "residual": [("run", 10), ("state", 1.01), ("run", 1), ("residual",), ("run", 5), ("run", 5), ("run", 5), ("residual",)],
     "output": [("run", 25), ("csv",), ("run", 25), ("state", 1.01), ("run", 3), ("run", 3), ("residual",)],
+    # lengths that come back often enough for a graph of their own, and one more
+    "returning": [("run", 2), ("run", 3)] * 5 + [("residual",)] + [("run", 2), ("run", 3)] * 40 + [("residual",), ("run", 2)],
     "chunks": [("run", 1), ("state", 1.01), ("run", 10), ("run", 10), ("residual",), ("run", 20), ("residual",)],
 }
 
