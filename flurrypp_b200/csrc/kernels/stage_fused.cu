@@ -429,9 +429,11 @@ __global__ void __launch_bounds__(Fz<ND, P, R>::NT, Fz<ND, P, R>::MINB)
 
   if constexpr (TMA) {
     __syncthreads();  // barrier object, sE
-    if (!mbar_wait_bounded(bar, 0, 1u << 22)) {
-      // give up: flag it, let the copies in flight land (bounded), leave
-      if (a.err) atomicOr(a.err, 1);
+    if (!__syncthreads_and(mbar_wait_bounded(bar, 0, 1u << 22))) {
+      // give up, the whole block or none of it (the barriers and the tile
+      // stores below need every thread): flag it, let the copies in flight
+      // land (bounded), leave
+      if (tid == 0 && a.err) atomicOr(a.err, 1);
       cp_async_wait<0>();
       mbar_wait_bounded(bar, 0, 1u << 22);
       return;
