@@ -35,37 +35,44 @@ struct Phys {
   int riemannType;    // 0 Rusanov, 1 Roe (2-D interior faces only)
 };
 
-// 1/x and sqrt(x) of a positive state value by Newton's method from the
-// hardware's approximation (relative error below 2^-20 in FP64, 2^-22 in
-// FP32; each step squares the error), the last step formed as a residual
-// correction, which leaves at most the last bit open.  Without the general
-// functions' branches for subnormal and huge arguments the chains of a
-// point's states overlap: they are the longest of a flux evaluation.  A root
-// below 1e-290 (FP32 1e-36), which no state reaches, is taken as zero; a
-// non-finite argument gives a non-finite result.
+// 1/x and sqrt(x) by Newton's method from the hardware's approximation
+// (relative error below 2^-20 in FP64, 2^-22 in FP32; each step squares the
+// error), the last step formed as a residual correction, which leaves at most
+// the last bit open (FP32: every mantissa gives the rounded value).  Without
+// the general functions' branches for subnormal and huge arguments the chains
+// of a point's states overlap: they are the longest of a flux evaluation.
+// Zeros, infinities, NaN and (root) negative arguments give what 1/x and
+// sqrt(x) give, by a select: a state that went wrong has to stay visible.
+// Subnormal results and arguments count as zero, and a root below 2^-963
+// (FP32 2^-119), which no state reaches, gives its argument back.
 __device__ __forceinline__ double recip(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double y0 = y, e = fma(-x, y, 1.0);  // NaN where y is 0, infinite or NaN
+  y = fma(y, e, y);
   y = fma(y, fma(-x, y, 1.0), y);
-  return fma(y, fma(-x, y, 1.0), y);
+  return e == e ? y : y0;
 }
 __device__ __forceinline__ float recip(float x) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return fmaf(y, fmaf(-x, y, 1.0f), y);
+  const float e = fmaf(-x, y, 1.0f);
+  return e == e ? fmaf(y, e, y) : y;
 }
 __device__ __forceinline__ double root(double x) {
   double r;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
   r = fma(0.5 * r, fma(-x * r, r, 1.0), r);
   const double s = x * r, h = 0.5 * r;
-  return x > 1e-290 ? fma(h, fma(-s, s, x), s) : 0.0;
+  const bool in = (unsigned)(__double2hiint(x) - 0x03c00000) < 0x7ff00000u - 0x03c00000u;
+  return x >= 0.0 && !in ? x : fma(h, fma(-s, s, x), s);
 }
 __device__ __forceinline__ float root(float x) {
   float r;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   const float s = x * r, h = 0.5f * r;
-  return x > 1e-36f ? fmaf(h, fmaf(-s, s, x), s) : 0.0f;
+  const bool in = (unsigned)(__float_as_int(x) - 0x04000000) < 0x7f800000u - 0x04000000u;
+  return x >= 0.0f && !in ? x : fmaf(h, fmaf(-s, s, x), s);
 }
 
 // Euler flux F[d][k] (reference: src/flux.cpp:37-76).
