@@ -205,7 +205,9 @@ __device__ __forceinline__ void roe2d(const R *UL, const R *UR, const R *n, R ga
   R lambdaP = fabs(unm + am);
   R lambdaM = fabs(unm - am);
   R eps = R(0.5) * (fabs(rhoUnL * rL - rhoUnR * rR) + fabs(root(gamma * pL * rL) - root(gamma * pR * rR)));
-  const R re = recip(eps);  // unused where eps is 0
+  // unused where eps is 0; a subnormal eps (flow at rest but for the tail of a
+  // disturbance) has no finite reciprocal, and the term it would scale is below it
+  const R re = eps > R(sizeof(R) == 4 ? 1.2e-38 : 2.3e-308) ? recip(eps) : R(0);
   if (lambda0 < R(2.) * eps) lambda0 = R(0.25) * lambda0 * lambda0 * re + eps;
   if (lambdaP < R(2.) * eps) lambdaP = R(0.25) * lambdaP * lambdaP * re + eps;
   if (lambdaM < R(2.) * eps) lambdaM = R(0.25) * lambdaM * lambdaM * re + eps;
