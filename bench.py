@@ -61,9 +61,9 @@ E2E_CASES = 4  # cases in flight in the end-to-end measurement (default of --e2e
 WORKLOAD = "3D Euler Taylor-Green vortex, 32^3 hexes, P=3, RK4, Rusanov, FP64 plain form"
 
 
-def profiled_traffic(kernel_tag: str):
-    """DRAM bytes per launch of a kernel from the committed ncu summary."""
-    p = os.path.join(ROOT, "profiles", "one_launch_stage.md")
+def profiled_traffic(kernel_tag: str, summary: str):
+    """DRAM bytes per launch of a kernel from a committed ncu summary."""
+    p = os.path.join(ROOT, "profiles", summary)
     try:
         for line in open(p):
             if line.startswith(kernel_tag + ":"):
@@ -282,6 +282,30 @@ def stage_bytes(s, wbytes):
     return E * (wbytes * (5 * nS * nF + 2 * nFp * nF + (nd * nd + 1) * nS + (nd + 1) * nFp) + 4 * nFp)
 
 
+def elem_bytes(s, wbytes):
+    """The same of the element launch of the two-kernel form: the common flux
+    (nFp nF) in place of the neighbours' traces, normals and areas."""
+    nS, nFp, nF, nd, E = s.nSpts, s.nFpts, s.nFields, s.nDims, s.nEles
+    return wbytes * E * (5 * nS * nF + 2 * nFp * nF + (nd * nd + 1) * nS)
+
+
+def stage_kernels(fb, s, wbytes, time_ms):
+    """Kernel times of the form the case's steps run in, and its dominant
+    kernel: one launch per stage, or (an explicit tile shape, short memory)
+    faces and elements.  time_ms(kernel) times one kernel of the case."""
+    real = "float" if wbytes == 4 else "double"
+    two = {"element_stage": time_ms("element_stage"), "faces": time_ms("faces")}
+    try:
+        ms = time_ms("stage")
+    except fb.FrError as e:
+        if e.code != fb.FR_ERR_UNSUPPORTED:
+            raise
+        return two, {"kernel": f"k_elem_tma<3, 3, {real}>", "kernel_ms": two["element_stage"],
+                     "algorithmic_bytes": elem_bytes(s, wbytes)}
+    return ({"stage": ms, "two_kernel_form": two},
+            {"kernel": f"k_fused_stage<3, 3, {real}>", "kernel_ms": ms, "algorithmic_bytes": stage_bytes(s, wbytes)})
+
+
 def kernel_ms(torch, stream, s, kernel, reps=20):
     s.bench_kernel(kernel, 2)
     return dev_ms(torch, stream, lambda: s.bench_kernel(kernel, reps)) / reps
@@ -296,12 +320,9 @@ def form_precision_tgv32(args, fb, torch, stream, dt):
     s.run(args.warmup)
     ms = dev_ms(torch, stream, lambda: s.run(args.steps))
     inf = s.info()
-    sm = kernel_ms(torch, stream, s, "stage")
-    km = kernel_ms(torch, stream, s, "element_stage")
-    fm = kernel_ms(torch, stream, s, "faces")
+    kms, top = stage_kernels(fb, s, 4, lambda k: kernel_ms(torch, stream, s, k))
     peak, _ = measured_peak_hbm()
-    eb = stage_bytes(s, 4)
-    ach = eb / (sm / 1e3) / 1e9
+    ach = top["algorithmic_bytes"] / (top["kernel_ms"] / 1e3) / 1e9
     del s
     # error after 200 steps vs the plain form, same initial state and dt
     runs = {}
@@ -318,10 +339,10 @@ def form_precision_tgv32(args, fb, torch, stream, dt):
         "value": dof * nrk * args.steps / (ms / 1e3), "unit": METRIC, "ms_per_step": ms / args.steps,
         "dtype": "f32 (FP64 dt, metrics at setup, norms)",
         "tile_variant": inf.tile_variant, "elems_per_block": inf.elems_per_block,
-        "kernels_ms": {"stage": sm, "two_kernel_form": {"element_stage": km, "faces": fm}},
-        "roofline": {"bound": "hbm", "kernel": "k_fused_stage<3, 3, float>",
+        "kernels_ms": kms,
+        "roofline": {"bound": "hbm", "kernel": top["kernel"],
                      "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
-                     "algorithmic_bytes": eb},
+                     "algorithmic_bytes": top["algorithmic_bytes"]},
         "error_vs_fp64": dict(steps=args.err_steps, **state_errors(runs[fb.FR_PREC_MIXED], runs[fb.FR_PREC_FP64])),
     }
 
@@ -874,16 +895,7 @@ def main():
     s.check_state()
 
     # dominant kernels timed alone (same stream)
-    kt = {}
-    for k in ("stage", "element_stage", "faces"):
-        s.bench_kernel(k, 2)
-        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        reps = 20
-        a.record(stream)
-        s.bench_kernel(k, reps)
-        b.record(stream)
-        torch.cuda.synchronize()
-        kt[k] = a.elapsed_time(b) / reps
+    kms, top = stage_kernels(fb, s, 8, lambda k: kernel_ms(torch, stream, s, k))
 
     # end to end through the C ABI with host buffers (pinned): every step
     # copies its case's state in from pinned host memory, advances it one RK
@@ -968,13 +980,15 @@ def main():
         e2e_copy_bound = whole_job_rate(world, dof, nrk, args.e2e_steps, ms_copy)
         peak, peak_kind = measured_peak_hbm()
         nF, nd = s.nFields, s.nDims
-        alg_bytes = stage_bytes(s, 8)
         inf = s.info()
         # face kernel: per face point read 2 slots, normal, dA L/R, U L/R;
         # write Fn L/R and the left wave speed
         nfp = inf.nFacePts
         face_bytes = nfp * (8 + 8 * nd + 16 + 2 * 8 * nF + 2 * 8 * nF + 8)
-        ach = alg_bytes / (kt["stage"] / 1e3) / 1e9
+        faces_ms = kms.get("two_kernel_form", kms)["faces"]
+        summary, tag = (("one_launch_stage.md", "one_launch_traffic_bytes") if "stage" in kms
+                        else ("fp64_stage_tgv32_p3.md", "traffic_bytes_per_launch"))
+        ach = top["algorithmic_bytes"] / (top["kernel_ms"] / 1e3) / 1e9
         out = {
             "metric": METRIC, "value": value, "unit": METRIC, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True,
@@ -986,15 +1000,13 @@ def main():
                     "copy_bound": e2e_copy_bound, "frac_of_copy_bound": e2e / e2e_copy_bound},
             "gpu_launches": launches,
             "roofline": {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
-                         "traffic": profiled_traffic("one_launch_traffic_bytes"),
-                         "traffic_source": "profiles/one_launch_stage.md (ncu, one launch)",
-                         "kernel": "k_fused_stage<3, 3, double>",
+                         "traffic": profiled_traffic(tag, summary),
+                         "traffic_source": f"profiles/{summary} (ncu, one launch)",
+                         "kernel": top["kernel"],
                          "tile_variant": inf.tile_variant, "elems_per_block": inf.elems_per_block,
-                         "kernel_ms": kt["stage"], "algorithmic_bytes": alg_bytes,
+                         "kernel_ms": top["kernel_ms"], "algorithmic_bytes": top["algorithmic_bytes"],
                          "peak_source": peak_kind},
-            "kernels_ms": {"stage": kt["stage"],
-                           "two_kernel_form": {"element_stage": kt["element_stage"], "faces": kt["faces"],
-                                               "faces_GBps": face_bytes / (kt["faces"] / 1e3) / 1e9}},
+            "kernels_ms": dict(kms, faces_GBps=face_bytes / (faces_ms / 1e3) / 1e9),
             "clocks": clk.summary(),
         }
         if world == 1 and not args.no_cpu_baseline:
