@@ -165,7 +165,9 @@ struct fr_case {
   bool mixed = false;
   // programmatic dependent launch for cases whose grids fit in about one wave
   // (a solution point per thread: 148 SMs x 1024 threads)
+  static constexpr long long kOneWavePoints = 148LL * 1024;
   bool usePdl = false;
+  long long finePoints = 0;  // solution points of the finest P-multigrid level
   int variant64 = 0;              // plain form: element tile variant in use
   std::vector<float> tuneMs64;    // plain form: element-stage ms per tile variant
   struct Fp32 {
@@ -414,6 +416,7 @@ struct fr_case {
   bool setup_device() {
     const fr_setup_opts &o = opts;
     size_t nU = (size_t)nS * E * nF, nUf = (size_t)nFp * E * nF;
+    if (!pmgCoarse) finePoints = (long long)nS * E;
     if (!alloc(U, nU)) return false;
     if (!mixed) {
       if (!alloc(U0, nU) || !alloc(acc, nU) || !alloc(Ufpts, nUf) || !alloc(Fn, nUf)) return false;
@@ -548,7 +551,7 @@ struct fr_case {
     }
     if (!alloc(devErr, 1)) return false;
     if (in.motion && !setup_motion()) return false;
-    usePdl = !opts.no_pdl && (long long)nS * E <= 148LL * 1024;
+    usePdl = !opts.no_pdl && (long long)nS * E <= kOneWavePoints;
     if (!mixed) {
       useTma = useTp && !opts.no_tma && build_tma(0);
       if (useTma && in.viscous) EB = frk::tma_elems_per_block<double>(nDims, in.order);
@@ -593,6 +596,7 @@ struct fr_case {
       L->in.order = P;
       L->mesh = mesh;
       L->pmgCoarse = true;
+      L->finePoints = finePoints;
       L->stream = stream;
       if (!L->setup(opts)) return fail(FR_ERR_SETUP, "P-multigrid level " + std::to_string(P) + ": " + L->err);
       std::vector<double> Uic;
@@ -1274,10 +1278,20 @@ struct fr_case {
 
   // One-launch stages: inviscid static cases with tensor-product operators
   // and an even number of stages, unless an option asks for another kernel.
+  // Not P-multigrid cases of one wave (those with programmatic launch): every
+  // CTA of a small case has boundaries, and they are served many at a time, when
+  // the wide CTAs (128 threads of 126 registers, two boundary states in a row)
+  // keep the other cases' CTAs out.  Channels, time of the two-kernel form over
+  // the one-launch form, FP64: 24 x 8 to 96 x 32 quads, P1 .. P4, one in flight
+  // 0.95 .. 1.24, three 0.81 .. 1.17 (mean 1.02), eight 0.74 .. 1.02, sixteen
+  // 0.51 .. 1.02 (mean 0.71); FP32 1.04 .. 1.29, 0.95 .. 1.27, 0.88 .. 1.16,
+  // 0.80 .. 1.33 (mean 0.96; 16 served requests 0.85).  At 160 x 53 P3 (136
+  // thousand points) eight in flight 1.00, from 200 x 66 on 1.11 .. 1.36 for any
+  // number.
   bool setup_fused() {
     const int n = in.order + 1, nLines = nS / n;
     if (!useTp || in.viscous || in.motion || nRK % 2 != 0 || opts.no_tma || opts.tile_variant >= 0 ||
-        (long long)nFp * E >= (1LL << 30))
+        (in.PMG && finePoints <= kOneWavePoints) || (long long)nFp * E >= (1LL << 30))
       return true;
     const int eb = mixed ? frk::fused_elems_per_block<float>(nDims, in.order)
                          : frk::fused_elems_per_block<double>(nDims, in.order);
