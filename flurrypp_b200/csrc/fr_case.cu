@@ -231,6 +231,7 @@ struct fr_case {
   // one part of a case split by a partition (fr_shard_*): the face points
   // the partition cuts; their right traces arrive in cut.recv before every
   // face pass (the shard packs and exchanges them for all parts)
+  bool splitPart = false;
   frk::CutTableT<double> cut;
   std::vector<int> cutPeer;  // peer part of every cut point (sorted by peer)
   // a part on its own rank (fr_part_create): the traces travel by NCCL
@@ -1290,7 +1291,7 @@ struct fr_case {
   // number.
   bool setup_fused() {
     const int n = in.order + 1, nLines = nS / n;
-    if (!useTp || in.viscous || in.motion || nRK % 2 != 0 || opts.no_tma || opts.tile_variant >= 0 ||
+    if (splitPart || !useTp || in.viscous || in.motion || nRK % 2 != 0 || opts.no_tma || opts.tile_variant >= 0 ||
         (in.PMG && finePoints <= kOneWavePoints) || (long long)nFp * E >= (1LL << 30))
       return true;
     const int eb = mixed ? frk::fused_elems_per_block<float>(nDims, in.order)
@@ -1363,7 +1364,7 @@ struct fr_case {
     fz.on = true;
     return true;
   }
-  bool fused_ok() const { return fz.on && cut.n == 0; }
+  bool fused_ok() const { return fz.on; }
 
   // One stage: -1 the residual alone (divF_out), else stage `st` of a step.
   // keepDivF / keepU0 / wave: the arrays a caller may look at after the call.
@@ -1592,6 +1593,7 @@ struct fr_case {
   // inviscid, static mesh, no P-multigrid (the creator checks).
   bool split_from(const fr_case &full, const std::vector<int> &part, int r, cudaStream_t st) {
     opts = full.opts;
+    splitPart = true;
     opts.no_pdl = 1;  // parts run in one stream with copies between their kernels
     in = full.in;
     nDims = full.nDims;

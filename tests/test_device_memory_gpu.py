@@ -1,0 +1,39 @@
+"""What a case takes of the device's memory: the tables of one-launch stages
+only where they are used and where they leave room for other cases."""
+import numpy as np
+import pytest
+
+import flurrypp_b200 as fb
+from flurrypp_b200.decks import write_deck
+
+pytestmark = pytest.mark.gpu
+
+MB = 1 << 20
+
+
+def box(tmp_path, n, order=3):
+    o = dict(nDims=len(n), order=order, meshType=1, dt=0.001)
+    for name, m in zip("xyz", n):
+        o.update({"n" + name: m, name + "min": 0, name + "max": 1.0})
+    return write_deck(str(tmp_path / "m.deck"), **o)
+
+
+def taken(make):
+    """(object, device bytes it took)."""
+    import torch
+
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    s = make()
+    return s, before - torch.cuda.mem_get_info()[0]
+
+
+def test_parts_of_a_split_case_take_no_tables(tmp_path):
+    d = box(tmp_path, (20, 20, 20))
+    for make in (lambda: fb.Solver(d), lambda: fb.Shard(d, 2)):  # the context's own memory
+        taken(make)
+    one, whole = taken(lambda: fb.Solver(d))
+    two, plain = taken(lambda: fb.Solver(d, tile_variant=0))
+    sh, parts = taken(lambda: fb.Shard(d, 2))
+    assert whole > 1.3 * plain  # the tables, which the parts leave out
+    assert parts < 1.1 * plain + 32 * MB
