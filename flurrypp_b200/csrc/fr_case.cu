@@ -347,6 +347,13 @@ struct fr_case {
     p = (T *)q;
     return true;
   }
+  // gives the newest buffer back (setup only; nothing may be using it)
+  void drop_last() {
+    cudaStreamSynchronize(stream);
+    if (allocs.back().fp32) note_fp32(allocs.back().p, allocs.back().bytes, false);
+    cudaFree(allocs.back().p);
+    allocs.pop_back();
+  }
   template <typename T>
   bool upload(T *&p, const std::vector<T> &h) {
     if (!alloc(p, h.size())) return false;
@@ -1297,16 +1304,19 @@ struct fr_case {
     const int eb = mixed ? frk::fused_elems_per_block<float>(nDims, in.order)
                          : frk::fused_elems_per_block<double>(nDims, in.order);
     const size_t nBlk = (E + eb - 1) / eb, lanes = nBlk * nLines * eb;
-    std::vector<int> lines(hLineF);
-    lines.insert(lines.end(), hLineOf.begin(), hLineOf.end());
-    if (!upload(fz.lineF, lines)) return false;
-    fz.lineOf = fz.lineF + hLineF.size();
     const bool ok = mixed ? setup_fused_as<float>(fz.f, lanes, eb, f32.U, f32.acc, f32.U0, f32.Ufpts, f32.JGinv,
                                                   f32.detJ, f32.ft)
                           : setup_fused_as<double>(fz.d, lanes, eb, U, acc, U0, Ufpts, JGinv, detJ, ft);
-    if (!ok) return false;
+    if (!ok) {  // an optimisation: without its memory or maps the two-kernel form runs
+      cudaGetLastError();
+      err.clear();
+      errCode = 0;
+      return true;
+    }
+    fz.on = true;
     return cuda_ok("one-launch stage setup");
   }
+  // false: no memory or no tensor maps; what it took is given back
   template <typename R>
   bool setup_fused_as(FusedDev<R> &z, size_t lanes, int eb, R *u, R *b, R *u0, R *uf, const R *jgi, const R *det,
                       const frk::FaceTableT<R> &table) {
@@ -1321,18 +1331,17 @@ struct fr_case {
     };
     const size_t oJ = take(lanes * n * nDims * nDims), oR = take(lanes * n), oN = take(lanes * 2 * nDims * (nDims + 1)),
                  oX = take(lanes * n * nF), oS = take(lanes * n * nF), oT = take(nUf),
-                 oB = take((lanes * 2 * nDims * sizeof(int) + sizeof(R) - 1) / sizeof(R));
+                 oB = take((lanes * 2 * nDims * sizeof(int) + sizeof(R) - 1) / sizeof(R)),
+                 oL = take(((hLineF.size() + hLineOf.size()) * sizeof(int) + sizeof(R) - 1) / sizeof(R));
     // a case that fills the memory keeps the two-kernel form
     size_t freeBytes = 0, allBytes = 0;
-    if (cudaMemGetInfo(&freeBytes, &allBytes) != cudaSuccess || total * sizeof(R) > freeBytes / 2) {
-      cudaGetLastError();
-      return true;
-    }
+    if (cudaMemGetInfo(&freeBytes, &allBytes) != cudaSuccess || total * sizeof(R) > freeBytes / 2) return false;
     R *pool = nullptr;
     if (!alloc(pool, total)) return false;
     z.jg = pool + oJ, z.rdet = pool + oR, z.nrm = pool + oN, z.X0 = pool + oX, z.S = pool + oS, z.Uf2 = pool + oT;
     fz.nb = reinterpret_cast<int *>(pool + oB);
-    frk::launch_fused_pack<R>(nDims, in.order, E, jgi, det, table, fz.lineOf, z.jg, z.rdet, fz.nb, z.nrm, stream);
+    fz.lineF = reinterpret_cast<int *>(pool + oL);
+    fz.lineOf = fz.lineF + hLineF.size();
     auto encode = tensor_map_encoder();
     const CUtensorMapDataType ty = sizeof(R) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     auto map = [&](CUtensorMap *m, void *p, int rows) {
@@ -1345,7 +1354,16 @@ struct fr_case {
     // rows of a tensor map start on 16-byte boundaries (2-D always do)
     fz.tma = encode && (size_t)E * nF * sizeof(R) % 16 == 0 && map(&z.U, u, nS) && map(&z.B, b, nS) &&
              map(&z.U0, u0, nS) && map(&z.Uf, uf, nFp) && map(&z.Uf2m, z.Uf2, nFp);
-    if (!fz.tma && nDims == 2) return fail(FR_ERR_CUDA, "tensor map");
+    std::vector<int> lines(hLineF);  // and, behind them, hLineOf
+    lines.insert(lines.end(), hLineOf.begin(), hLineOf.end());
+    if ((!fz.tma && nDims == 2) ||
+        cudaMemcpyAsync(fz.lineF, lines.data(), lines.size() * sizeof(int), cudaMemcpyHostToDevice, stream) !=
+            cudaSuccess ||
+        cudaStreamSynchronize(stream) != cudaSuccess) {
+      drop_last();
+      return false;
+    }
+    frk::launch_fused_pack<R>(nDims, in.order, E, jgi, det, table, fz.lineOf, z.jg, z.rdet, fz.nb, z.nrm, stream);
     frk::FusedArgsT<R> &a = z.a;
     a.E = E;
     a.S = z.S;
@@ -1361,7 +1379,6 @@ struct fr_case {
     a.ph = ph;
     for (int i = 0; i < n * n; i++) a.D[i] = (R)hD[i];
     for (int i = 0; i < 2 * n; i++) a.E1[i] = (R)hE1[i], a.EFn1[i] = (R)hEF[i], a.C[i] = (R)hLC[i];
-    fz.on = true;
     return true;
   }
   bool fused_ok() const { return fz.on; }
