@@ -1333,9 +1333,12 @@ struct fr_case {
                  oX = take(lanes * n * nF), oS = take(lanes * n * nF), oT = take(nUf),
                  oB = take((lanes * 2 * nDims * sizeof(int) + sizeof(R) - 1) / sizeof(R)),
                  oL = take(((hLineF.size() + hLineOf.size()) * sizeof(int) + sizeof(R) - 1) / sizeof(R));
-    // a case that fills the memory keeps the two-kernel form
+    // The tables are nearly half of what a case holds otherwise (3-D P3 FP64: 17
+    // KB a hex beside 37).  They may take an eighth of the memory that is free:
+    // up to four equal cases then fit beside each other as without tables, and a
+    // case alone has them up to 1.0 million such hexes on 180 GB.
     size_t freeBytes = 0, allBytes = 0;
-    if (cudaMemGetInfo(&freeBytes, &allBytes) != cudaSuccess || total * sizeof(R) > freeBytes / 2) return false;
+    if (cudaMemGetInfo(&freeBytes, &allBytes) != cudaSuccess || total * sizeof(R) > freeBytes / 8) return false;
     R *pool = nullptr;
     if (!alloc(pool, total)) return false;
     z.jg = pool + oJ, z.rdet = pool + oR, z.nrm = pool + oN, z.X0 = pool + oX, z.S = pool + oS, z.Uf2 = pool + oT;

@@ -37,3 +37,41 @@ def test_parts_of_a_split_case_take_no_tables(tmp_path):
     sh, parts = taken(lambda: fb.Shard(d, 2))
     assert whole > 1.3 * plain  # the tables, which the parts leave out
     assert parts < 1.1 * plain + 32 * MB
+
+
+def test_a_second_case_fits_beside_the_first(tmp_path):
+    """With memory for two cases and not for both of their tables, both are set
+    up, and run as they do with memory to spare (2-D: bit for bit)."""
+    import torch
+
+    d = box(tmp_path, (256, 256))
+    U = None
+    ends = []
+
+    def end(s):
+        nonlocal U
+        if U is None:
+            U = np.array([1.0, 0.3, 0.1, 2.0]) * (1 + np.random.default_rng(7).uniform(-0.01, 0.01, s.shape))
+        s.set_state(U)
+        s.run(3)
+        return s.get_state()
+
+    for v in (-1, 0):  # the kernels of both forms are loaded
+        ends.append(end(fb.Solver(d, tile_variant=v)))
+    one, plain = taken(lambda: fb.Solver(d, tile_variant=0))
+    two, whole = taken(lambda: fb.Solver(d))
+    del one, two
+    tables = whole - plain
+    assert tables > 0.2 * plain
+    torch.cuda.empty_cache()
+    left = 2 * plain + tables * 6 // 10
+    rest = torch.empty(torch.cuda.mem_get_info()[0] - left, dtype=torch.uint8, device="cuda")
+    try:
+        both = [fb.Solver(d), fb.Solver(d)]
+        ends += [end(s) for s in both]
+        del both
+    finally:
+        del rest
+        torch.cuda.empty_cache()
+    for e in ends[1:]:
+        assert np.array_equal(e, ends[0])
