@@ -357,8 +357,8 @@ struct fr_case {
   template <typename T>
   bool upload(T *&p, const std::vector<T> &h) {
     if (!alloc(p, h.size())) return false;
-    cudaError_t e = cudaMemcpyAsync(p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    // from pageable memory the call returns once the source has been read
+    const cudaError_t e = cudaMemcpyAsync(p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, stream);
     if (e != cudaSuccess) {
       err = std::string("cudaMemcpy: ") + cudaGetErrorString(e);
       errCode = FR_ERR_CUDA;
@@ -1115,6 +1115,19 @@ struct fr_case {
   // changes the speed only, never the result.
   bool autotune_tiles() {
     const bool tc = frk::tc_supported(nDims, in.order) && !opts.no_tensor_cores;
+    const int nv = frk::tma_variants(true) + (tc ? 1 : 0);
+    int forced = opts.tile_variant;
+    f32.tuneMs.assign(nv, -1.0f);
+    if (forced >= nv) return fail(FR_ERR_ARG, "tile_variant out of range");
+    // small cases: launches of a few microseconds time as noise, so the
+    // choice is fixed (the first shape, not timed) and identical cases stay
+    // identical
+    if (forced < 0 && (long long)nS * E < kTuneMinPoints) {
+      f32.useTma = build_tma32(0);
+      f32.variant = 0;
+      if (f32.useTma) EB = frk::tma_elems_per_block<float>(nDims, in.order, 0);
+      return true;
+    }
     if (tc && !f32.tcOps) {
       const double *g[3] = {op.grad[0].data(), op.grad[1].data(), nDims == 3 ? op.grad[2].data() : nullptr};
       const double *x[3] = {op.extFn[0].data(), op.extFn[1].data(), nDims == 3 ? op.extFn[2].data() : nullptr};
@@ -1122,13 +1135,6 @@ struct fr_case {
       if (!frk::tc_pack_ops(nDims, in.order, g, x, op.corr.data(), op.ext.data(), blob) || !upload(f32.tcOps, blob))
         return fail(FR_ERR_CUDA, "tensor-core operator upload");
     }
-    const int nv = frk::tma_variants(true) + (tc ? 1 : 0);
-    int forced = opts.tile_variant;
-    f32.tuneMs.assign(nv, -1.0f);
-    if (forced >= nv) return fail(FR_ERR_ARG, "tile_variant out of range");
-    // small cases: launches of a few microseconds time as noise, so the
-    // choice is fixed (the first shape) and identical cases stay identical
-    if (forced < 0 && (long long)nS * E < kTuneMinPoints) forced = 0;
     int best = -1;
     float bestMs = 0.0f;
     const int tpEB = EB;
@@ -1336,9 +1342,12 @@ struct fr_case {
     // The tables are nearly half of what a case holds otherwise (3-D P3 FP64: 17
     // KB a hex beside 37).  They may take an eighth of the memory that is free:
     // up to four equal cases then fit beside each other as without tables, and a
-    // case alone has them up to 1.0 million such hexes on 180 GB.
+    // case alone has them up to 1.0 million such hexes on 180 GB.  (Up to 8 MB are
+    // tried without asking, which costs 0.1 to 0.4 ms.)
     size_t freeBytes = 0, allBytes = 0;
-    if (cudaMemGetInfo(&freeBytes, &allBytes) != cudaSuccess || total * sizeof(R) > freeBytes / 8) return false;
+    if (total * sizeof(R) > (8u << 20) &&
+        (cudaMemGetInfo(&freeBytes, &allBytes) != cudaSuccess || total * sizeof(R) > freeBytes / 8))
+      return false;
     R *pool = nullptr;
     if (!alloc(pool, total)) return false;
     z.jg = pool + oJ, z.rdet = pool + oR, z.nrm = pool + oN, z.X0 = pool + oX, z.S = pool + oS, z.Uf2 = pool + oT;
@@ -1361,8 +1370,7 @@ struct fr_case {
     lines.insert(lines.end(), hLineOf.begin(), hLineOf.end());
     if ((!fz.tma && nDims == 2) ||
         cudaMemcpyAsync(fz.lineF, lines.data(), lines.size() * sizeof(int), cudaMemcpyHostToDevice, stream) !=
-            cudaSuccess ||
-        cudaStreamSynchronize(stream) != cudaSuccess) {
+            cudaSuccess) {
       drop_last();
       return false;
     }
@@ -1462,8 +1470,8 @@ struct fr_case {
     const int nv = frk::tma_variants(false);
     int forced = opts.tile_variant;
     if (forced >= nv) return fail(FR_ERR_ARG, "tile_variant out of range for the plain form");
-    if (forced < 0 && (long long)nS * E < kTuneMinPoints) forced = 0;  // small: fixed choice
     tuneMs64.assign(nv, -1.0f);
+    if (forced < 0 && (long long)nS * E < kTuneMinPoints) return true;  // small: the first shape, as built, not timed
     int best = -1;
     float bestMs = 0.0f;
     cudaEvent_t e0, e1;
