@@ -366,6 +366,15 @@ struct fr_case {
     }
     return true;
   }
+  // device bytes held, the coarse levels' included: buffers of 1 MB and more
+  // come in pages of 2 MB, smaller ones share them
+  size_t device_bytes() const {
+    size_t n = 0;
+    for (auto &b : allocs) n += b.bytes < (1u << 20) ? (b.bytes + 511) / 512 * 512 : (b.bytes + (2u << 20) - 1) / (2u << 20) * (2u << 20);
+    for (auto &L : levels)
+      if (L) n += L->device_bytes();
+    return n;
+  }
   bool cuda_ok(const char *what) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
@@ -2709,6 +2718,12 @@ int fr_get_info(fr_case *c, fr_info *info) {
     cudaMemcpy(&info->time, c->timeAcc, sizeof(double), cudaMemcpyDeviceToHost);
     cudaMemcpy(&info->dt, c->dt, sizeof(double), cudaMemcpyDeviceToHost);
   }
+  return FR_OK;
+}
+
+int fr_device_bytes(const fr_case *c, size_t *bytes) {
+  if (!c || !bytes) return FR_ERR_ARG;
+  *bytes = c->device_bytes();
   return FR_OK;
 }
 

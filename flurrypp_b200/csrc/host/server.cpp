@@ -43,6 +43,9 @@ struct Request {
   // in flight
   fr_case *c = nullptr;
   size_t bytes = 0;
+  size_t need = 0;    // bytes it was found to need, waiting for room (form needForm)
+  int needForm = -1;
+  bool lean = false;  // without the tables of one-launch stages, to fit the budget
   int steps = 0;
   int pending = 0;  // steps issued and not yet seen complete
   int nFields = 0;
@@ -77,15 +80,12 @@ struct fr_server {
   std::vector<long long> inflight;
   std::string err;
 
-  // device bytes of a case, from its sizes (setup allocations; P-multigrid
-  // levels add their share)
-  static size_t case_bytes(fr_case *c) {
-    fr_info inf;
-    if (fr_get_info(c, &inf) != FR_OK) return 0;
-    size_t nU = (size_t)inf.nSpts * inf.nEles * inf.nFields, nUf = (size_t)inf.nFpts * inf.nEles * inf.nFields;
-    size_t words = nU * (3 + inf.nRKSteps + 3) + nUf * 2 + (size_t)inf.nDims * inf.nDims * inf.nSpts * inf.nEles +
-                   (size_t)inf.nFpts * inf.nEles * (inf.nDims + 2) + (size_t)inf.nFacePts * (inf.nDims + 4);
-    return words * sizeof(double) * 2;  // coarse P levels and tables: at most as much again
+  // Device bytes a request holds while it runs: what its case allocated; a
+  // refining one goes on in FP64, with at most twice the bytes of its FP32 case.
+  static size_t case_bytes(const Request &r, const fr_case *c) {
+    size_t n = 0;
+    fr_device_bytes(c, &n);
+    return r.refine && r.fp32 ? 2 * n : n;
   }
 
   static fr_case *create(Request &r, int device, int prec, int &st) {
@@ -93,6 +93,7 @@ struct fr_server {
     fr_setup_opts_default(&o);
     o.device = device;
     o.precision = prec;
+    if (r.lean) o.tile_variant = 0;
     fr_case *c = nullptr;
     st = r.hasMesh ? fr_create_with_mesh(r.deck.c_str(), &r.mesh, &o, &c)
                    : fr_create_from_deck(r.deck.c_str(), &o, &c);
@@ -112,22 +113,35 @@ struct fr_server {
     if (fr_get_info(r.c, &inf) != FR_OK) return false;
     std::vector<double> U((size_t)inf.nSpts * inf.nEles * inf.nFields);
     if (fr_get_state(r.c, U.data(), U.size()) != FR_OK) return false;
-    int st = FR_OK;
-    fr_case *c = create(r, device, FR_PREC_FP64, st);
-    if (st != FR_OK || fr_set_state(c, U.data(), U.size()) != FR_OK) {
+    const auto in_fp64 = [&]() -> fr_case * {
+      int st = FR_OK;
+      fr_case *c = create(r, device, FR_PREC_FP64, st);
+      if (st == FR_OK) return c;
+      fr_destroy(c);
+      return nullptr;
+    };
+    fr_case *c = in_fp64();
+    size_t held = 0;
+    if (c && fr_device_bytes(c, &held) == FR_OK && held > r.bytes && !r.lean) {  // stay within what was admitted
+      fr_destroy(c);
+      r.lean = true;
+      c = in_fp64();
+    }
+    if (!c) return false;
+    if (fr_set_state(c, U.data(), U.size()) != FR_OK) {
       fr_destroy(c);
       return false;
     }
     fr_destroy(r.c);
     r.c = c;
-    const size_t b = case_bytes(c);
+    r.fp32 = false;
+    const size_t b = case_bytes(r, c);
     {
       std::lock_guard<std::mutex> lk(mu);
       inflightBytes += b;
       inflightBytes -= r.bytes;
     }
     r.bytes = b;
-    r.fp32 = false;
     r.form = FR_PREC_FP64;
     r.stepsFp32 = r.steps;
     return true;
@@ -140,18 +154,30 @@ struct fr_server {
     r.refine = precision == FR_PREC_MIXED_REFINE;
     r.form = r.refine ? FR_PREC_MIXED : precision;
     r.fp32 = r.form == FR_PREC_MIXED;
+    const int want = r.refine ? FR_PREC_MIXED_REFINE : r.form;
+    if (r.needForm != want) r.lean = false;
+    if (r.needForm == want && !inflight.empty() && inflightBytes + r.need > budget) return false;  // no room yet
     int st = FR_OK;
-    fr_case *c = create(r, device, r.form, st);
-    if (st == FR_OK) st = fr_init_solution(c, r.icKind, r.icPrm.empty() ? nullptr : r.icPrm.data(), (int)r.icPrm.size());
-    if (st != FR_OK) {
-      r.status = 3;
-      r.code = st;
-      r.error = c ? fr_last_error(c) : "create failed";
-      fr_destroy(c);
-      queue.pop_front();
-      return true;
+    fr_case *c = nullptr;
+    size_t b = 0;
+    for (;;) {
+      c = create(r, device, r.form, st);
+      if (st == FR_OK) st = fr_init_solution(c, r.icKind, r.icPrm.empty() ? nullptr : r.icPrm.data(), (int)r.icPrm.size());
+      if (st != FR_OK) {
+        r.status = 3;
+        r.code = st;
+        r.error = c ? fr_last_error(c) : "create failed";
+        fr_destroy(c);
+        queue.pop_front();
+        return true;
+      }
+      b = case_bytes(r, c);
+      if (b <= budget || r.lean) break;
+      fr_destroy(c);  // more than the whole budget: once more without the tables
+      r.lean = true;
     }
-    size_t b = case_bytes(c);
+    r.need = b;
+    r.needForm = want;
     if (!inflight.empty() && inflightBytes + b > budget) {
       fr_destroy(c);  // no room yet: wait for a retirement
       return false;

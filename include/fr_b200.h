@@ -116,6 +116,8 @@ int fr_create_with_mesh(const char *deck_path, const fr_mesh *mesh, const fr_set
 void fr_destroy(fr_case *c);
 const char *fr_last_error(const fr_case *c);
 int fr_get_info(fr_case *c, fr_info *info);
+/* Device memory the case holds, its coarse P-multigrid levels included. */
+int fr_device_bytes(const fr_case *c, size_t *bytes);
 
 /* Kernels of the case run on this stream (a cudaStream_t; NULL = default). */
 int fr_set_stream(fr_case *c, void *stream);

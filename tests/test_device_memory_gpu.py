@@ -75,3 +75,41 @@ def test_a_second_case_fits_beside_the_first(tmp_path):
         torch.cuda.empty_cache()
     for e in ends[1:]:
         assert np.array_equal(e, ends[0])
+
+
+@pytest.mark.parametrize("prec", [fb.FR_PREC_FP64, fb.FR_PREC_MIXED])
+def test_server_counts_what_its_cases_hold(tmp_path, prec):
+    """A P-multigrid case large enough for one-launch stages: the bytes the
+    server counts are those the device gave (to the 2 MB of its pages), and a
+    budget below them and above what the case needs without its tables is
+    served without them."""
+    import time
+
+    import torch
+
+    d = write_deck(str(tmp_path / "p.deck"), nDims=2, order=2, meshType=1, nx=132, ny=130, xmin=0, xmax=1, ymin=0, ymax=1,
+                   dtType=2, CFL=0.3, PMG=1, lowOrder=0, smoothSteps=2, uBound=0.35)
+    plain, whole = (taken(lambda: fb.Solver(d, precision=prec, tile_variant=v))[1] for v in (0, -1))
+    assert whole > 1.15 * plain
+
+    def serve(budget, max_steps, ic=(fb.IC_UNIFORM, ())):
+        srv = fb.Server(budget_bytes=budget, max_inflight=2, check_every=10, precision=prec)
+        return srv, srv.submit(d, ic=ic, tol=1e-30, max_steps=max_steps)
+
+    srv, rid = serve(8 << 30, 20)  # loads the kernels
+    srv.wait(rid, 120)
+    srv.close()
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    srv, rid = serve(8 << 30, 10 ** 6)
+    t0, counted = time.time(), 0
+    while counted == 0 and time.time() - t0 < 60:
+        counted = srv.stats()["inflight_bytes"]
+    held = before - torch.cuda.mem_get_info()[0]
+    srv.cancel(rid)
+    srv.close()
+    assert counted >= 0.9 * held - 8 * MB, (counted, held)
+    srv, rid = serve(counted - 1, 20)
+    srv.wait(rid, 120)
+    assert srv.poll(rid)["status"] == 2
+    srv.close()
