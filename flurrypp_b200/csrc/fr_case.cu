@@ -1456,13 +1456,13 @@ struct fr_case {
       fused_launch<double>(fz.d, st, U, acc, U0, Ufpts, nullptr, keepDivF ? divF[0] : nullptr,
                            pmgSource ? src : nullptr, keepU0, wave);
   }
-  // Fn_fpts of the last evaluation, where one-launch stages did not store it
   // new traces of a state the caller changed: first Fn_fpts of the last
   // evaluation, if it is still to be formed from the traces replaced here
   void renew_traces() {
     if (!fnOld) ensure_fn();
     extrapolate();
   }
+  // Fn_fpts of the last evaluation, where one-launch stages did not store it
   void ensure_fn() {
     if (!fnStale) return;
     if (mixed)

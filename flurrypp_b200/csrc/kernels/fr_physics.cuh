@@ -1,8 +1,9 @@
 // Point-wise physics on the device: Euler flux, common (Riemann) fluxes,
 // boundary ghost states, LDG viscous flux.  Each function restates the
 // reference's arithmetic in the same operation order, so the FP64 form
-// differs from the reference CPU build only by FMA contraction and operator
-// application order (<= a few ulp per point).
+// differs from the reference CPU build only by FMA contraction, operator
+// application order and, in the fluxes, one reciprocal per divisor multiplied
+// in place of a division per term (<= a few ulp per point).
 #pragma once
 #include <cuda_runtime.h>
 

@@ -63,8 +63,9 @@ typedef struct fr_setup_opts {
   int device;                  /* CUDA device ordinal; -1: host-side setup only */
   int generic_kernels;         /* 1: use the general sparse-operator element kernel */
   int no_tma;                  /* 1: tensor-product element kernel without TMA tiles */
-  int tile_variant;            /* -1 (default): one-launch stages where they apply; 0 and up: the two-kernel
-                                  form with that element tile shape (-1: autotuned at setup);
+  int tile_variant;            /* -1 (default): one-launch stages where they apply, else the two-kernel form with
+                                  the tile shape timed at setup (small cases: the first); 0 and up: the
+                                  two-kernel form with that element tile shape;
                                   the last variant of 2-D orders 1..4 is the tensor-core (tcgen05) kernel */
   int no_tensor_cores;         /* 1: leave the tensor-core variant out of the autotuner's choice */
   int no_pdl;                  /* 1: no programmatic dependent launch (used for small cases by default) */
@@ -95,7 +96,7 @@ typedef struct fr_info {
   double time, dt;
   long long launches; /* kernels this case has launched (graph replays counted per kernel) */
   int tensor_kernels; /* 0 general, 1 tensor-product, 2 tensor-product with TMA tiles */
-  int tile_variant;   /* precision form: element tile shape in use (-1: none) */
+  int tile_variant;   /* element tile shape of the two-kernel form (-1: none) */
   int elems_per_block;
 } fr_info;
 
@@ -153,8 +154,8 @@ int fr_update(fr_case *c, int pmg_source);
 int fr_pmg_cycle(fr_case *c);
 
 /* n steps of the reference's driver loop: update(), then, with PMG 1, the
- * V-cycle (src/flurry.cpp:162-170).  The steady-state step is captured once
- * as a CUDA graph and replayed. */
+ * V-cycle (src/flurry.cpp:162-170).  Steady-state steps are replayed as CUDA
+ * graphs of one step, of ten, and of a smaller number that has come back often. */
 int fr_run(fr_case *c, int nsteps);
 
 /* CFL time step (solver::calcDt, src/solver.cpp:447-468); *dt = global dt. */
