@@ -42,38 +42,44 @@ struct Phys {
 // the last bit open (FP32: every mantissa gives the rounded value).  Without
 // the general functions' branches for subnormal and huge arguments the chains
 // of a point's states overlap: they are the longest of a flux evaluation.
-// Zeros, infinities, NaN and (root) negative arguments give what 1/x and
-// sqrt(x) give, by a select: a state that went wrong has to stay visible.
-// Subnormal results and arguments count as zero, and a root below 2^-963
-// (FP32 2^-119), which no state reaches, gives its argument back.
+// A state that went wrong stays visible: recip of zeros, infinities and NaN is
+// NaN, root of zeros, infinities, NaN and negative arguments is what sqrt
+// gives.  Subnormal reciprocals count as zero, and an argument of root below
+// 1e-290 (FP32 1e-36), which no state reaches, is given back.
 __device__ __forceinline__ double recip(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double y0 = y, e = fma(-x, y, 1.0);  // NaN where y is 0, infinite or NaN
-  y = fma(y, e, y);
   y = fma(y, fma(-x, y, 1.0), y);
-  return e == e ? y : y0;
+  return fma(y, fma(-x, y, 1.0), y);
 }
 __device__ __forceinline__ float recip(float x) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  const float e = fmaf(-x, y, 1.0f);
-  return e == e ? fmaf(y, e, y) : y;
+  return fmaf(y, fmaf(-x, y, 1.0f), y);
 }
-__device__ __forceinline__ double root(double x) {
+__device__ __forceinline__ double newton_root(double x) {
   double r;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
   r = fma(0.5 * r, fma(-x * r, r, 1.0), r);
   const double s = x * r, h = 0.5 * r;
-  const bool in = (unsigned)(__double2hiint(x) - 0x03c00000) < 0x7ff00000u - 0x03c00000u;
-  return x >= 0.0 && !in ? x : fma(h, fma(-s, s, x), s);
+  return fma(h, fma(-s, s, x), s);
 }
-__device__ __forceinline__ float root(float x) {
+__device__ __forceinline__ float newton_root(float x) {
   float r;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   const float s = x * r, h = 0.5f * r;
-  const bool in = (unsigned)(__float_as_int(x) - 0x04000000) < 0x7f800000u - 0x04000000u;
-  return x >= 0.0f && !in ? x : fmaf(h, fmaf(-s, s, x), s);
+  return fmaf(h, fmaf(-s, s, x), s);
+}
+template <typename R>
+__device__ __forceinline__ R root(R x) {
+  const R v = newton_root(x);
+  const bool in = x > R(sizeof(R) == 4 ? 1e-36 : 1e-290) && x <= R(sizeof(R) == 4 ? 3.4e38 : 1.79e308);
+  return x >= R(0) && !in ? x : v;
+}
+// of an argument that is not negative; infinity gives NaN (two selects less)
+template <typename R>
+__device__ __forceinline__ R root_of_nonnegative(R x) {
+  return x > R(sizeof(R) == 4 ? 1e-36 : 1e-290) ? newton_root(x) : x;
 }
 
 // Euler flux F[d][k] (reference: src/flux.cpp:37-76).
@@ -155,7 +161,7 @@ __device__ __forceinline__ R rusanov(const R *UL, const R *UR, const R *n, R gam
   }
   R csqL = fmax(gam * L.p * L.rinv, R(0.0));
   R csqR = fmax(gam * Rt.p * Rt.rinv, R(0.0));
-  const R cL = root(csqL), cR = root(csqR);
+  const R cL = root_of_nonnegative(csqL), cR = root_of_nonnegative(csqR);
   R eigL = fabs(vnL) + cL;
   R eigR = fabs(vnR) + cR;
   R eig = fmax(eigL, eigR);
