@@ -635,9 +635,9 @@ __global__ void k_norm_total(int nF, long long nSE, int E, const R *__restrict__
     if (resType == 1)
       r += fabs(d) * w[(int)(j / E)];
     else if (resType == 2)
-      r += d * d * recip(detJ[j]) * w[(int)(j / E)];
+      r += d * d / detJ[j] * w[(int)(j / E)];
     else  // a NaN anywhere makes the maximum NaN (fmax would drop it)
-      r = nan_max(fabs(d) * recip(detJ[j]), r);
+      r = nan_max(fabs(d) / detJ[j], r);
   }
   fold(r);
   if (j0 == 0) {
