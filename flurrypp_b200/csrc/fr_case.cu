@@ -354,11 +354,20 @@ struct fr_case {
     cudaFree(allocs.back().p);
     allocs.pop_back();
   }
+  bool inSetup = false;                 // setup_device: one synchronisation at its end
+  std::vector<std::vector<char>> kept;  // small uploads' sources until then
   template <typename T>
   bool upload(T *&p, const std::vector<T> &h) {
     if (!alloc(p, h.size())) return false;
-    // from pageable memory the call returns once the source has been read
-    const cudaError_t e = cudaMemcpyAsync(p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, stream);
+    const size_t bytes = h.size() * sizeof(T);
+    const void *src = h.data();
+    const bool small = inSetup && bytes > 0 && bytes <= 64 * 1024;
+    if (small) {  // a copy that lives until the setup's synchronisation
+      kept.emplace_back((const char *)src, (const char *)src + bytes);
+      src = kept.back().data();
+    }
+    cudaError_t e = cudaMemcpyAsync(p, src, bytes, cudaMemcpyHostToDevice, stream);
+    if (e == cudaSuccess && !small) e = cudaStreamSynchronize(stream);  // h may go
     if (e != cudaSuccess) {
       err = std::string("cudaMemcpy: ") + cudaGetErrorString(e);
       errCode = FR_ERR_CUDA;
@@ -433,6 +442,7 @@ struct fr_case {
   bool setup_device() {
     const fr_setup_opts &o = opts;
     size_t nU = (size_t)nS * E * nF, nUf = (size_t)nFp * E * nF;
+    inSetup = true;
     if (!pmgCoarse) finePoints = (long long)nS * E;
     if (!alloc(U, nU)) return false;
     if (!mixed) {
@@ -596,6 +606,8 @@ struct fr_case {
     }
     if (!setup_fused()) return false;  // last: it does without where memory is short
     if (cudaStreamSynchronize(stream) != cudaSuccess) return fail(FR_ERR_CUDA, "setup sync");
+    inSetup = false;
+    kept.clear();
     return cuda_ok("setup");
   }
 
@@ -1379,7 +1391,8 @@ struct fr_case {
     lines.insert(lines.end(), hLineOf.begin(), hLineOf.end());
     if ((!fz.tma && nDims == 2) ||
         cudaMemcpyAsync(fz.lineF, lines.data(), lines.size() * sizeof(int), cudaMemcpyHostToDevice, stream) !=
-            cudaSuccess) {
+            cudaSuccess ||
+        cudaStreamSynchronize(stream) != cudaSuccess) {
       drop_last();
       return false;
     }
